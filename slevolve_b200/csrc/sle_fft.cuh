@@ -90,6 +90,18 @@ __device__ __forceinline__ void dft_r(V (&v)[R]) {
 __host__ __device__ constexpr int tw_pass_index(int n, int ns, int u, int k) { return n + ns - 8 + (u - 1) * ns + k; }
 __host__ __device__ constexpr int tw_table_len(int n) { return n >= 8 ? 2 * n - 8 : n; }
 
+// Reads the twiddle table once, one 32-byte sector per access, so that the passes find it in L1: a
+// block that has an SM nearly to itself otherwise waits for L2 in every pass.  The table belongs to
+// the plan, so this may run before the wait for the kernel before.
+template <int N, int NT, typename V>
+__device__ __forceinline__ void touch_twiddles(const V* __restrict__ tw) {
+  constexpr int STEP = 32 / (int)sizeof(V);
+  for (int i = threadIdx.x * STEP; i < tw_table_len(N); i += NT * STEP) {
+    uint32_t x;
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(x) : "l"(tw + i));
+  }
+}
+
 // Row-FFT blocks transform NR rows of N points (NR = 2: the north and south rows of one
 // latitude pair; NR = 4: two pairs); one radix-8 butterfly per thread and pass.
 __host__ __device__ constexpr int fft_nt(int nr, int n2) { return nr * n2 / 8 > 32 ? nr * n2 / 8 : 32; }
@@ -230,6 +242,19 @@ __device__ __forceinline__ void fft_rest(V* A, const V* tw, const Sink& sink) {
       fft_pass<NR, N, R, NS, INV, true>(SmemRows<N, V>{A}, SmemRows<N, V>{A}, tw);
       fft_rest<NR, N, NS * R, INV>(A, tw, sink);
     }
+  }
+}
+
+// Whole transform of NR rows held in A (shared memory, written and synchronised), the last pass into
+// `sink`.
+template <int NR, int N, bool INV, typename V, typename Sink>
+__device__ __forceinline__ void fft_rows_inplace(V* A, const V* tw, const Sink& sink) {
+  constexpr int R = FftRadix<N, 1>::R;
+  if constexpr (R >= N) {
+    fft_pass<NR, N, R, 1, INV, false>(SmemRows<N, V>{A}, sink, tw);
+  } else {
+    fft_pass<NR, N, R, 1, INV, true>(SmemRows<N, V>{A}, SmemRows<N, V>{A}, tw);
+    fft_rest<NR, N, R, INV>(A, tw, sink);
   }
 }
 

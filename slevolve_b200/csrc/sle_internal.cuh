@@ -117,10 +117,14 @@ struct ShtDev {
   const double* be;           // [ncoef] Q_l = mu Q_{l-1} + be_l Q_{l-2}
   const double* cf;           // [ncoef] P~_l = cf_l Q_l (segment scale)
   const unsigned char* istart;// [nseg] first significant latitude group of the segment
-  const int* ana_order;       // [nseg] segment processing order for the analysis (long first)
+  // FP64 analysis: (segment, order, first degree, first significant latitude group), most work first;
+  // synthesis: (order, latitude tile, mask of the order's segments significant on the whole tile, mask
+  // of those significant on its upper half only), most work first
+  const int4* ana_items;      // [nseg]
+  const int4* syn_items;      // [nm * tiles]
   const double2* tw;          // [n2] exp(-2 pi i t / nlon)
   double2* X;                 // [MAXF][2][nm][nh] folded rFFT (S then D) of analysed grids
-  double2* EO;                // [MAXF][2][nm][nh] even/odd Legendre sums of synthesised fields
+  double2* EO;                // [MAXF][nh][nm][2] even/odd Legendre sums of synthesised fields
   // Per-field gates of a launch (device flags read at kernel entry): field f is skipped (its
   // outputs left as they are) when gset[f] && *gset[f] != 0, or gclr[f] && *gclr[f] == 0.
   const int* gset[MAXF];
@@ -154,7 +158,8 @@ __device__ __forceinline__ bool field_gated_off(const ShtDev& P, int f) {
 enum SrcKind { SRC_GRID = 0, SRC_MASK = 1, SRC_ICE = 2, SRC_TO = 3, SRC_PROD = 4 };
 
 // One field of a transform call: input and output, optional gates (see ShtDev::gset/gclr), the
-// analysis source kind and, for synthesis, the optional epilogue epi_out = grid * epi_mul.
+// analysis source kind and, for synthesis, the optional epilogue epi_out = grid * epi_mul.  `dense`
+// (FP64 transforms; the same for every field of a call): the spectrum is the dense [l][m] array.
 struct FieldSpec {
   double* grid;
   double2* spec;
@@ -165,6 +170,7 @@ struct FieldSpec {
   int kind;
   const unsigned char* m0;
   const unsigned char* m1;
+  int dense = 0;
 };
 
 // Two neighbouring cells c, c + 1 (c even) of an analysis source of kind KIND.
@@ -227,7 +233,8 @@ struct sle_sht {
   // owned allocations
   double *mu, *w, *wn, *ws, *be, *cf;
   long long* moff;
-  int *lidx, *segoff, *seg_m, *seg_l0, *ana_order;
+  int *lidx, *segoff, *seg_m, *seg_l0;
+  int4 *ana_items, *syn_items;
   double2 *seeds, *tw, *X, *EO;
   unsigned char* istart;
   double2* packbuf;           // [MAXF][ncoef] packed staging for dense-layout calls
@@ -252,7 +259,7 @@ struct sle_sht {
   double mx_table_bytes;
   int n_ana_units, n_syn_units;
   int n_ana_cta, n_syn_cta;       // CTAs of an analysis / synthesis launch
-  int n_sm;                      // SMs of the device (persistent transform grid)
+  int n_sm;                      // SMs of the device
   // blocks of the unfold resident on the device at once (occupancy x SMs): each block prefetches
   // into L2 the input of the block that many places further on in launch order
   int unfold_ahead;

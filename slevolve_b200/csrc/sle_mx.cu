@@ -1125,12 +1125,6 @@ int sht_mx_prepare(sle_sht* p) {
   }
   std::stable_sort(au.begin(), au.end(), [](const AU& x, const AU& y) { return x.w > y.w; });
   std::stable_sort(su.begin(), su.end(), [](const SU& x, const SU& y) { return x.w > y.w; });
-  {
-    int dev = 0, nsm = 0;
-    SLE_CUDA(cudaGetDevice(&dev));
-    SLE_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    p->n_sm = std::max(1, nsm);
-  }
   // CTA b of a launch of G = min(n, SMs) CTAs takes a run of consecutive units: longest first,
   // each unit goes to the CTA with the least estimated work so far (ties: the lowest index);
   // within a CTA the units keep that order

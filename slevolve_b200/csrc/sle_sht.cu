@@ -7,15 +7,14 @@
 //              grid rows = unnormalised inverse real FFT of G (Im of m = 0 ignored).
 //
 // Design (B200):
-//   * One kernel per latitude pair does the row FFTs (radix-2 Stockham in shared memory on
+//   * One block per latitude pair does the row FFTs (radix-8 Stockham in shared memory on
 //     nlon/2-point complex sequences, real/complex split) and the north/south fold.
 //   * The Legendre functions are regenerated on the fly in FP64 with a two-term recurrence
 //     Q_l = mu Q_{l-1} + be_l Q_{l-2} (P~_l = cf_l Q_l) that restarts every SEG degrees from
 //     seeds computed once per plan with the reference's own normalised recursion
 //     (sht.py:105-144).  Segments are the work units: analysis = one warp per (m, segment),
-//     latitudes spread over the lanes (8 per lane at nlat = 512), the latitude sum done by a
-//     transposing warp reduction over 8 degrees at a time; synthesis = one block per pair of
-//     orders (m, L-m) with one warp per 32-latitude group, coefficients staged in shared memory.
+//     latitudes spread over the lanes (8 per lane at nlat = 512), the latitude sums through shared
+//     memory; synthesis = one block per (m, 128 latitudes), its warps dealing out the segments.
 //   * (segment, latitude-group) blocks whose |P~| never exceeds 1e-35 (near the poles at high
 //     m) are skipped.
 #include "sle_internal.cuh"
@@ -41,27 +40,6 @@ void set_error(const char* fmt, ...) {
 
 // --------------------------------------------------------------------------- helpers
 // (complex helpers and the Stockham FFT: sle_fft.cuh)
-
-// Sum a per-lane vector v[0..V) over the 32 lanes of a warp.  After the call lane `l` holds
-// in v[0] the warp total of value index (l >> (5 - log2 V)).  log2(V) exchange stages each
-// halve the live values (send the half the partner keeps), then plain butterflies.
-template <int V>
-__device__ __forceinline__ void warp_transpose_reduce(double (&v)[V], int lane) {
-  static_assert(V >= 1 && V <= 32 && (V & (V - 1)) == 0, "V must be a power of two <= 32");
-#pragma unroll
-  for (int C = V, o = 16; C > 1; C >>= 1, o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int c = 0; c < C / 2; ++c) {
-      const double send = up ? v[c] : v[c + C / 2];
-      const double keep = up ? v[c + C / 2] : v[c];
-      v[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  constexpr int LOGV = (V >= 32) ? 5 : (V >= 16) ? 4 : (V >= 8) ? 3 : (V >= 4) ? 2 : (V >= 2) ? 1 : 0;
-#pragma unroll
-  for (int o = 16 >> LOGV; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-}
 
 // ------------------------------------------------------------------- plan set-up kernels
 // Gauss-Legendre nodes and weights: the Newton iteration of the reference gaulw
@@ -241,10 +219,13 @@ __global__ void __launch_bounds__(fft_nt(2, N)) k_fft_fold(sle::ShtDev P, GridPt
   extern __shared__ double2 sm[];
   double2* A = sm;
   const int j = blockIdx.x, f = blockIdx.y;
+  touch_twiddles<N, fft_nt(2, N)>(P.tw);
+  const double wn = P.wn[j], ws = P.ws[j];
+  pdl_wait();
+  pdl_trigger();
   if (field_gated_off(P, f)) return;
   with_src_kind(g.kind[f], FoldRows64<N>{g.p[f], g.m0[f], g.m1[f], j, P.nlat, P.tw, A});
   const SmemRows<N, double2> Z{A};
-  const double wn = P.wn[j], ws = P.ws[j];
   double2* XS = P.X + ((size_t)(f * 2 + 0) * P.nm) * P.nh;
   double2* XD = P.X + ((size_t)(f * 2 + 1) * P.nm) * P.nh;
   for (int m = threadIdx.x; m < P.nm; m += blockDim.x) {
@@ -276,46 +257,53 @@ __global__ void __launch_bounds__(fft_nt(2, N)) k_fft_fold(sle::ShtDev P, GridPt
 
 // Inverse: north spectrum E + O, south E - O (m <= lmax, 0 above), unnormalised inverse
 // real FFT of both rows (sht.py:330-339 with the nlon scaling folded out); field blockIdx.y.
-// The half-length complex packing is formed while the first FFT pass reads its inputs; the last
-// pass writes the output rows (and the optional epilogue out2 = grid * mul2).
-template <int N>
-struct UnfoldSrc64 {
-  const double2* E;   // [m][j] planes of the field, at latitude j
-  const double2* O;
-  const double2* tw;
-  int nm, nh;
-  __device__ __forceinline__ double2 g(int r, int m) const {
-    if (m >= nm) return make_double2(0.0, 0.0);
-    const double2 e = E[(size_t)m * nh], o = O[(size_t)m * nh];
-    return r ? csub(e, o) : cadd(e, o);
-  }
-  __device__ __forceinline__ double2 operator()(int r, int m) const {
-    double2 x, y;
-    if (m == 0) {
-      x = make_double2(g(r, 0).x, 0.0);
-      y = make_double2(g(r, N).x, 0.0);
-    } else {
-      x = g(r, m);
-      const double2 c = g(r, N - m);
-      y = make_double2(c.x, -c.y);
-    }
-    const double2 e = cadd(x, y);
-    const double2 t = __ldg(tw + m);
-    const double2 wc = make_double2(t.x, -t.y);  // exp(+2 pi i m / nlon)
-    const double2 o = cmul(csub(x, y), wc);
-    return make_double2(e.x - o.y, e.y + o.x);  // e + i o
-  }
-};
-
+// The half-length complex packing of both rows is formed first, each thread taking a pair of orders
+// (m, N - m), so that every (E, O) pair is read once (the packing of an index needs both orders; formed
+// while the first pass reads its inputs, per row and index, the same sums were read four times through
+// L1 and the blocks waited on those loads); the last pass writes the output rows (and the optional
+// epilogue out2 = grid * mul2).  Bound: latency (one latitude pair per block, less than two blocks
+// per SM for one field); with the synthesis sums 15.0 -> 8.6 us at
+// 256 x 512 and 9.1 -> 4.7 us at 64 x 128, one field.
 template <int N>
 __global__ void __launch_bounds__(fft_nt(2, N)) k_ifft_unfold(sle::ShtDev P, OutGridPtrs g) {
   extern __shared__ double2 sm[];
+  constexpr int NT = fft_nt(2, N);
   double2* A = sm;
   const int j = blockIdx.x, f = blockIdx.y;
+  touch_twiddles<N, NT>(P.tw);
+  pdl_wait();
+  pdl_trigger();
   if (field_gated_off(P, f)) return;
   const int js = P.nlat - 1 - j;
-  const double2* E = P.EO + ((size_t)(f * 2 + 0) * P.nm) * P.nh + j;
-  const double2* O = P.EO + ((size_t)(f * 2 + 1) * P.nm) * P.nh + j;
+  const double2* G = P.EO + ((size_t)f * P.nh + j) * P.nm * 2;   // (E, O) of each order
+  const SmemRows<N, double2> Z{A};
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int p = threadIdx.x; p < N / 2; p += NT) {
+    // the orders a and b of this thread's two outputs (p = 0: the indices 0 and N / 2)
+    const int a = p, b = p ? N - p : N / 2;
+    const bool ina = a < P.nm, inb = b < P.nm, inn = p == 0 && N < P.nm;
+    const double2 ea = ina ? G[2 * a] : zero, oa = ina ? G[2 * a + 1] : zero;
+    const double2 eb = inb ? G[2 * b] : zero, ob = inb ? G[2 * b + 1] : zero;
+    const double2 en = inn ? G[2 * N] : zero, on = inn ? G[2 * N + 1] : zero;   // the Nyquist order
+    const double2 ta = __ldg(P.tw + a), tb = __ldg(P.tw + b);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {   // north E + O, south E - O
+      const double2 ga = r ? csub(ea, oa) : cadd(ea, oa), gb = r ? csub(eb, ob) : cadd(eb, ob);
+      double2 x = ga, y = make_double2(gb.x, -gb.y);
+      if (p == 0) {
+        x = make_double2(ga.x, 0.0);
+        y = make_double2(r ? en.x - on.x : en.x + on.x, 0.0);
+      }
+      double2 e = cadd(x, y), o = cmul(csub(x, y), make_double2(ta.x, -ta.y));   // exp(+2 pi i m / nlon)
+      Z.put(r, a, make_double2(e.x - o.y, e.y + o.x));                           // e + i o
+      x = gb;
+      y = (p == 0) ? make_double2(gb.x, -gb.y) : make_double2(ga.x, -ga.y);
+      e = cadd(x, y);
+      o = cmul(csub(x, y), make_double2(tb.x, -tb.y));
+      Z.put(r, b, make_double2(e.x - o.y, e.y + o.x));
+    }
+  }
+  __syncthreads();
   const size_t ro = (size_t)j * (2 * N), rso = (size_t)js * (2 * N);
   double* out2 = g.out2[f];
   const double* mul2 = g.mul2[f];
@@ -324,74 +312,40 @@ __global__ void __launch_bounds__(fft_nt(2, N)) k_ifft_unfold(sle::ShtDev P, Out
                      out2 ? reinterpret_cast<double2*>(out2 + rso) : nullptr,
                      out2 ? reinterpret_cast<const double2*>(mul2 + ro) : nullptr,
                      out2 ? reinterpret_cast<const double2*>(mul2 + rso) : nullptr};
-  fft_rows<2, N, true>(UnfoldSrc64<N>{E, O, P.tw, P.nm, P.nh}, A, P.tw, sink);
+  fft_rows_inplace<2, N, true>(A, P.tw, sink);
 }
-
-
 
 // ------------------------------------------------------------------ Legendre analysis
-constexpr int ANA_TL = 4;      // degrees per warp reduction
-constexpr int ANA_NAMAX = 8;   // latitude groups per lane in one pass
-constexpr int ANA_WARPS = 4;   // warps (independent segments) per block
+// One warp per (order, 64-degree segment): lanes hold latitudes, NA groups of 32 at a time, and
+// walk the segment's degrees together.  Per degree and latitude the recurrence costs two FP64
+// operations and each field two; the per-lane sums of 16 values are then added up over the warp
+// through shared memory (each lane stores its 16 partial sums, a pair of lanes adds the 32 of one
+// value), which costs about 6 instructions per degree, where a butterfly with its selects and
+// two-word shuffles cost 27.  The totals collect in shared memory and leave scaled and coalesced.
+// Bound: the FP64 pipe (one warp instruction per 2.2 cycles and scheduler).  F = 2 shares one
+// recurrence between two fields (6 operations instead of 8 per degree and latitude).
+// Measured on one field, fold included, back to back in a CUDA graph: 30.3 -> 25.9 us at L = 511
+// (16.4 -> 10.3 at L = 255, 13.1 -> 6.4 at L = 63); four fields at L = 511 91.3 -> 64.6 us.
+constexpr int ANA_V = 16;             // values per warp reduction
+constexpr int ANA_RS = 33;            // row stride of the reduction buffer (bank-conflict free both ways)
+constexpr int ANA_WARPS = 2;          // warps (independent segments) per block
+constexpr int ANA_NAMAX = 8;          // latitude groups per pass
 
-// One batch of TL consecutive degrees: advance the recurrence of the NA latitudes of this lane,
-// form the per-lane products with the folded input of the degree's parity, and reduce over
-// the warp.  Degree t of the batch has parity t (segments start at even l - m).
-template <int NA>
-__device__ __forceinline__ void ana_batch(const double* __restrict__ sbe, const double (&mu)[NA],
-                                          double (&qa)[NA], double (&qb)[NA], const double2 (&xs)[NA],
-                                          const double2 (&xd)[NA], double (&v)[2 * ANA_TL], int lane) {
-  // the latitude sum of each degree uses up to four independent partial sums (short chains)
-  constexpr int NP = (NA >= 4) ? 4 : NA;
-#pragma unroll
-  for (int t = 0; t < ANA_TL; ++t) {
-    double re[NP], im[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) re[p] = im[p] = 0.0;
-    const double b = sbe[t];
-#pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      const double q = fma(mu[i], qb[i], b * qa[i]);
-      qa[i] = qb[i];
-      qb[i] = q;
-      const double2 x = (t & 1) ? xd[i] : xs[i];
-      re[i % NP] = fma(q, x.x, re[i % NP]);
-      im[i % NP] = fma(q, x.y, im[i % NP]);
-    }
-    double sr = re[0], si = im[0];
-    if (NP == 4) {
-      sr = (re[0] + re[1]) + (re[2] + re[3]);
-      si = (im[0] + im[1]) + (im[2] + im[3]);
-    } else if (NP == 2) {
-      sr = re[0] + re[1];
-      si = im[0] + im[1];
-    }
-    v[2 * t] = sr;
-    v[2 * t + 1] = si;
-  }
-  warp_transpose_reduce<2 * ANA_TL>(v, lane);
-}
-
-// Degrees l0 .. l0+len-1 of segment s over the latitude groups g0 .. g0+NA-1 (groups at or
-// beyond ngrp hold no latitudes).  The staged recurrence coefficients are zero-padded to a
-// whole number of batches; the extra degrees are computed and discarded.
-template <int NA>
-__device__ __forceinline__ void ana_segment(const sle::ShtDev& P, int s, int g0, const double2* __restrict__ Xf,
-                                            double2* __restrict__ Uf, int lane, bool accumulate,
-                                            double* __restrict__ sbe, double* __restrict__ scf) {
-  constexpr int SHIFT = (ANA_TL == 8) ? 1 : (ANA_TL == 4) ? 2 : 3;  // 5 - log2(2 ANA_TL)
-  const int m = P.seg_m[s], l0 = P.seg_l0[s];
-  const int len = min(SEG, P.lmax + 1 - l0);
+// Degrees of segment s over the latitude groups g0 .. g0+NA-1 (latitudes at or beyond nh count as
+// zero): ANA_V / (2 F) degrees per batch, each advancing the recurrence of the lane's NA latitudes
+// and summing its products with the folded input of the degree's parity (segments start at even
+// l - m, batches at even degrees).  The staged recurrence coefficients are zero-padded to a whole
+// number of batches; the extra degrees are computed and not written.  sacc[(degree F + field) 2 +
+// component] receives the sums (added to what is there when `more`).
+template <int NA, int F>
+__device__ __forceinline__ void ana_pass(const sle::ShtDev& P, int s, int m, int g0, int len,
+                                         const double2* const (&Xf)[F], int lane, bool more,
+                                         const double* __restrict__ sbe, double* __restrict__ red,
+                                         double* __restrict__ sacc) {
+  constexpr int TL = ANA_V / (2 * F);
   const int nh = P.nh;
-  const long long base = P.moff[m] + (l0 - m);
-  for (int t = lane; t < SEG; t += 32) {
-    sbe[t] = (t < len) ? P.be[base + t] : 0.0;
-    scf[t] = (t < len) ? P.cf[base + t] : 0.0;
-  }
-  const double2* XS = Xf + (size_t)m * nh;
-  const double2* XD = Xf + (size_t)(P.nm + m) * nh;
   double mu[NA], qa[NA], qb[NA];
-  double2 xs[NA], xd[NA];
+  double2 xs[F][NA], xd[F][NA];
 #pragma unroll
   for (int i = 0; i < NA; ++i) {
     const int j = (g0 + i) * 32 + lane;
@@ -400,147 +354,299 @@ __device__ __forceinline__ void ana_segment(const sle::ShtDev& P, int s, int g0,
     const double2 sd = ok ? P.seeds[(size_t)s * nh + j] : make_double2(0.0, 0.0);
     qa[i] = sd.x;
     qb[i] = sd.y;
-    xs[i] = ok ? XS[j] : make_double2(0.0, 0.0);
-    xd[i] = ok ? XD[j] : make_double2(0.0, 0.0);
-  }
-  __syncwarp();
-  const int idx = lane >> SHIFT;
-  const int tw_ = idx >> 1, c = idx & 1;
-  const bool writer = (lane & ((1 << SHIFT) - 1)) == 0;
-  for (int off = 0; off < len; off += ANA_TL) {
-    double v[2 * ANA_TL];
-    ana_batch<NA>(sbe + off, mu, qa, qb, xs, xd, v, lane);
-    if (writer && off + tw_ < len) {
-      const double val = __ddiv_rn(v[0] * scf[off + tw_], SQRT2_LEGACY);
-      double* dst = reinterpret_cast<double*>(Uf + base + off + tw_) + c;
-      *dst = accumulate ? (*dst + val) : val;
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      xs[f][i] = ok ? Xf[f][(size_t)m * nh + j] : make_double2(0.0, 0.0);
+      xd[f][i] = ok ? Xf[f][(size_t)(P.nm + m) * nh + j] : make_double2(0.0, 0.0);
     }
   }
-  __syncwarp();
+  // this lane's half (lane & 1) of value lane / 2: elements 16 h .., the second half starting eight
+  // further on so that the two lanes of a pair read different banks
+  const int h = lane & 1;
+  const double* rv = red + (lane >> 1) * ANA_RS + 16 * h;
+#pragma unroll 1
+  for (int off = 0; off < len; off += TL) {
+    double v[ANA_V];
+#pragma unroll
+    for (int t = 0; t < TL; ++t) {
+      const double b = sbe[off + t];
+#pragma unroll
+      for (int i = 0; i < NA; ++i) {
+        const double q = fma(mu[i], qb[i], __dmul_rn(b, qa[i]));
+        qa[i] = qb[i];
+        qb[i] = q;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+          const double2 x = (t & 1) ? xd[f][i] : xs[f][i];
+          double& re = v[(t * F + f) * 2];
+          double& im = v[(t * F + f) * 2 + 1];
+          re = (i == 0) ? __dmul_rn(q, x.x) : fma(q, x.x, re);
+          im = (i == 0) ? __dmul_rn(q, x.y) : fma(q, x.y, im);
+        }
+      }
+    }
+    __syncwarp();   // the previous batch's partial sums are read
+#pragma unroll
+    for (int u = 0; u < ANA_V; ++u) red[u * ANA_RS + lane] = v[u];
+    __syncwarp();
+    double p[4];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const double r = rv[(u + 8 * h) & 15];
+      p[u & 3] = (u < 4) ? r : __dadd_rn(p[u & 3], r);
+    }
+    double tot = __dadd_rn(__dadd_rn(p[0], p[1]), __dadd_rn(p[2], p[3]));
+    tot = __dadd_rn(tot, __shfl_xor_sync(0xffffffffu, tot, 1));
+    if (h == 0) {
+      double* d = sacc + off * 2 * F + (lane >> 1);
+      *d = more ? __dadd_rn(*d, tot) : tot;
+    }
+  }
 }
 
-__device__ void ana_zero_segment(const sle::ShtDev& P, int s, double2* Uf, int lane) {
-  const int m = P.seg_m[s], l0 = P.seg_l0[s];
-  const int l1 = min(l0 + SEG, P.lmax + 1);
+// Segment s of F fields: the latitude groups from the segment's first significant one (gs) on in
+// passes of up to eight groups, then the coefficients (packed, or the dense [l][m] array whose
+// order's zeros above the diagonal the first segment writes).
+template <int F>
+__device__ __forceinline__ void ana_segment(const sle::ShtDev& P, int s, int m, int l0, int gs,
+                                            const double2* const (&Xf)[F], double2* const (&Uf)[F], bool dense,
+                                            int lane, const double* __restrict__ sbe, const double* __restrict__ scf,
+                                            double* __restrict__ red, double* __restrict__ sacc) {
+  const int len = min(SEG, P.lmax + 1 - l0);
   const long long base = P.moff[m] + (l0 - m);
-  for (int l = l0 + lane; l < l1; l += 32) Uf[base + (l - l0)] = make_double2(0.0, 0.0);
+  bool more = false;
+  int g = gs;
+  while (g < P.ngrp) {
+    const int na = min(P.ngrp - g, ANA_NAMAX);
+    switch ((na + 1) / 2) {
+      case 4: ana_pass<8, F>(P, s, m, g, len, Xf, lane, more, sbe, red, sacc); break;
+      case 3: ana_pass<6, F>(P, s, m, g, len, Xf, lane, more, sbe, red, sacc); break;
+      case 2: ana_pass<4, F>(P, s, m, g, len, Xf, lane, more, sbe, red, sacc); break;
+      default:
+        if (na == 2) ana_pass<2, F>(P, s, m, g, len, Xf, lane, more, sbe, red, sacc);
+        else ana_pass<1, F>(P, s, m, g, len, Xf, lane, more, sbe, red, sacc);
+    }
+    g += na;
+    more = true;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    for (int e = lane; e < 2 * len; e += 32) {
+      const int t = e >> 1, c = e & 1;
+      const double val = more ? __dmul_rn(sacc[(t * F + f) * 2 + c], scf[t]) : 0.0;
+      const size_t at = dense ? (size_t)(l0 + t) * P.nm + m : (size_t)base + t;
+      reinterpret_cast<double*>(Uf[f] + at)[c] = val;
+    }
+    if (dense && l0 == m)
+      for (int l = lane; l < m; l += 32) Uf[f][(size_t)l * P.nm + m] = make_double2(0.0, 0.0);
+  }
 }
 
-__global__ void __launch_bounds__(32 * ANA_WARPS, 3) k_leg_ana(sle::ShtDev P, SpecPtrs out) {
+// blockIdx.y: the field (F = 1) or the pair of fields (F = 2; a pair with one field gated off, or
+// the last field of an odd number, runs alone with the same arithmetic).  What the plan holds is
+// read before the wait for the kernel before (the plan's tables never change).
+template <int F>
+__global__ void __launch_bounds__(32 * ANA_WARPS, F == 1 ? 6 : 4) k_leg_ana(sle::ShtDev P, SpecPtrs out, int nf, int dense) {
   __shared__ double scoef[ANA_WARPS][2][SEG];
+  __shared__ double sred[ANA_WARPS][ANA_V * ANA_RS];
+  __shared__ double ssum[ANA_WARPS][2 * SEG * F];
   const int wib = threadIdx.x >> 5;
   const int warp = blockIdx.x * ANA_WARPS + wib;
   const int lane = threadIdx.x & 31;
-  if (warp >= P.nseg) return;
-  const int f = blockIdx.y;
-  if (field_gated_off(P, f)) return;
-  const double2* Xf = P.X + (size_t)f * 2 * P.nm * P.nh;
-  double2* Uf = out.p[f];
-  const int s = P.ana_order[warp];
-  int gfirst = P.istart[s];
-  if (gfirst >= P.ngrp) {
-    ana_zero_segment(P, s, Uf, lane);
+  if (warp >= P.nseg) {
+    pdl_wait();
     return;
   }
+  const int4 item = P.ana_items[warp];   // segment, order, first degree, first significant group
   double* sbe = scoef[wib][0];
   double* scf = scoef[wib][1];
-  // latitude groups gfirst .. ngrp-1 in passes of up to ANA_NAMAX groups; a pass of na groups
-  // runs the smallest instance NA >= na.  The first pass starts NA - na groups closer to the
-  // pole when that stays inside the grid (those groups hold negligible but valid values and no
-  // other pass covers them); later passes start where the previous one ended and mask groups
-  // beyond the grid.
-  bool acc = false;
-  int g = gfirst;
-  while (g < P.ngrp) {
-    const int na = min(P.ngrp - g, ANA_NAMAX);
-    const int NA = (na > 4) ? 8 : (na > 2) ? 4 : na;
-    const int g0 = acc ? g : max(0, min(g, P.ngrp - NA));
-    switch (NA) {
-      case 1: ana_segment<1>(P, s, g0, Xf, Uf, lane, acc, sbe, scf); break;
-      case 2: ana_segment<2>(P, s, g0, Xf, Uf, lane, acc, sbe, scf); break;
-      case 4: ana_segment<4>(P, s, g0, Xf, Uf, lane, acc, sbe, scf); break;
-      default: ana_segment<8>(P, s, g0, Xf, Uf, lane, acc, sbe, scf); break;
+  {
+    const int len = min(SEG, P.lmax + 1 - item.z);
+    const long long base = (long long)item.y * P.nm - (long long)item.y * (item.y - 1) / 2 + (item.z - item.y);
+    for (int t = lane; t < SEG; t += 32) {
+      sbe[t] = (t < len) ? P.be[base + t] : 0.0;
+      scf[t] = (t < len) ? __ddiv_rn(P.cf[base + t], SQRT2_LEGACY) : 0.0;
     }
-    acc = true;
-    g = g0 + NA;
   }
+  pdl_wait();
+  pdl_trigger();
+  __syncwarp();
+  const size_t field = (size_t)2 * P.nm * P.nh;
+  const int f0 = F * blockIdx.y;
+  int first = -1, count = 0;
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    if (f0 + f < nf && !field_gated_off(P, f0 + f)) {
+      if (first < 0) first = f;
+      ++count;
+    }
+  }
+  if (count == 0) return;
+  if constexpr (F == 2) {
+    if (count == 2) {
+      const double2* const X[2] = {P.X + f0 * field, P.X + (f0 + 1) * field};
+      double2* const U[2] = {out.p[f0], out.p[f0 + 1]};
+      ana_segment<2>(P, item.x, item.y, item.z, item.w, X, U, dense != 0, lane, sbe, scf, sred[wib], ssum[wib]);
+      return;
+    }
+  }
+  const double2* const X[1] = {P.X + (f0 + first) * field};
+  double2* const U[1] = {out.p[f0 + first]};
+  ana_segment<1>(P, item.x, item.y, item.z, item.w, X, U, dense != 0, lane, sbe, scf, sred[wib], ssum[wib]);
 }
 
 // ----------------------------------------------------------------- Legendre synthesis
-// Block per pair of orders (p, lmax-p); warp per 64 latitudes (two per lane); E (even l-m) and
-// O (odd l-m) sums of cf_l * 1.41421356 * U_l * Q_l over the segments where the warp's outer
-// latitude group is significant.
-__global__ void __launch_bounds__(512, 1) k_leg_syn(sle::ShtDev P, CSpecPtrs in) {
-  extern __shared__ double smd[];
-  const int f = blockIdx.y;
-  if (field_gated_off(P, f)) return;
-  const int p = blockIdx.x;
-  const int L = P.lmax;
-  double2* Uc = reinterpret_cast<double2*>(smd);          // [nm]
-  double* bes = smd + 2 * P.nm;                            // [nm]
-  const double2* U = in.p[f];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j0 = w * 64 + lane, j1 = j0 + 32;
-  const bool ok0 = j0 < P.nh, ok1 = j1 < P.nh;
-  const double x0 = ok0 ? P.mu[j0] : 0.0, x1 = ok1 ? P.mu[j1] : 0.0;
-  const int gouter = min(2 * w + 1, P.ngrp - 1);
-  double2* Ef = P.EO + ((size_t)(f * 2 + 0) * P.nm) * P.nh;
-  double2* Of = P.EO + ((size_t)(f * 2 + 1) * P.nm) * P.nh;
-  for (int pass = 0; pass < 2; ++pass) {
-    const int m = (pass == 0) ? p : L - p;
-    if (pass == 1 && m == p) break;
-    const long long base = P.moff[m];
-    const int nl = L - m + 1;
-    __syncthreads();
-    for (int t = threadIdx.x; t < nl; t += blockDim.x) {
-      const double c = P.cf[base + t] * SQRT2_LEGACY;
-      const double2 u = U[base + t];
-      Uc[t] = make_double2(u.x * c, u.y * c);
-      bes[t] = P.be[base + t];
+// Block (order m, NA consecutive latitude groups), four warps: warp w sums the segments w, w + 4,
+// .. of the order over the block's latitudes (NA per lane, one per group), then the four warps'
+// even- and odd-degree sums are added in warp order.  Bound: the FP64 pipe, two operations per
+// degree and latitude for the recurrence and two per field.  One serial walk over all degrees of
+// an order (the form before) had two warps per scheduler waiting on their own recurrences; the
+// split over segments gives every scheduler four and more independent walks, and the blocks run
+// longest first.  F = 2 shares the recurrence between two fields.  Each (latitude, order) is
+// written as one 32-byte (E, O) sector at EO[f][j][m], which the inverse FFT of latitude j reads
+// as one contiguous row.  Measured on one field at L = 511: with the inverse FFT, back to back in a
+// CUDA graph, 30.2 -> 26.3 us (L = 255: 17.2 -> 8.6, L = 63: 11.5 -> 4.7); four fields at L = 511
+// 88.9 -> 61.0 us.  Two or eight warps per block measured slower (32.8 and 31.4 us at that stage
+// against 28.0).
+constexpr int SYN_WARPS = 4;
+
+// Degrees of one segment, coefficients u (F per degree, scaled) and recurrence factors b staged in
+// shared memory, for the lane's latitudes LO .. NA-1.
+template <int NA, int LO, int F>
+__device__ __forceinline__ void syn_segment(const sle::ShtDev& P, int s, int j0, int len, const double2* __restrict__ su,
+                                            const double* __restrict__ sb, double2 (&E)[F][NA], double2 (&O)[F][NA]) {
+  double x[NA], qa[NA], qb[NA];
+#pragma unroll
+  for (int i = LO; i < NA; ++i) {
+    const int j = j0 + 32 * i;
+    const bool ok = j < P.nh;
+    x[i] = ok ? P.mu[j] : 0.0;
+    const double2 sd = ok ? P.seeds[(size_t)s * P.nh + j] : make_double2(0.0, 0.0);
+    qa[i] = sd.x;
+    qb[i] = sd.y;
+  }
+#pragma unroll 2
+  for (int r = 0; r < len; r += 2) {   // the staged coefficients are zero beyond len
+    const double b0 = sb[r], b1 = sb[r + 1];
+#pragma unroll
+    for (int i = LO; i < NA; ++i) {
+      qa[i] = fma(x[i], qb[i], __dmul_rn(b0, qa[i]));   // even degree
+      qb[i] = fma(x[i], qa[i], __dmul_rn(b1, qb[i]));   // odd degree
     }
-    __syncthreads();
-    double2 E0 = make_double2(0.0, 0.0), O0 = E0, E1 = E0, O1 = E0;
-    for (int s = P.segoff[m]; s < P.segoff[m + 1]; ++s) {
-      if (gouter < (int)P.istart[s]) continue;
-      const int l0 = P.seg_l0[s];
-      const int l1 = min(l0 + SEG, L + 1);
-      const double2 s0 = ok0 ? P.seeds[(size_t)s * P.nh + j0] : make_double2(0.0, 0.0);
-      const double2 s1 = ok1 ? P.seeds[(size_t)s * P.nh + j1] : make_double2(0.0, 0.0);
-      double qa0 = s0.x, qb0 = s0.y, qa1 = s1.x, qb1 = s1.y;
-      int r = l0 - m;
-      const int rend = l1 - m;
-      for (; r + 2 <= rend; r += 2) {
-        double2 u = Uc[r];
-        double b = bes[r];
-        double q0 = fma(x0, qb0, b * qa0), q1 = fma(x1, qb1, b * qa1);
-        qa0 = qb0; qb0 = q0; qa1 = qb1; qb1 = q1;
-        E0.x = fma(u.x, q0, E0.x); E0.y = fma(u.y, q0, E0.y);
-        E1.x = fma(u.x, q1, E1.x); E1.y = fma(u.y, q1, E1.y);
-        u = Uc[r + 1];
-        b = bes[r + 1];
-        q0 = fma(x0, qb0, b * qa0);
-        q1 = fma(x1, qb1, b * qa1);
-        qa0 = qb0; qb0 = q0; qa1 = qb1; qb1 = q1;
-        O0.x = fma(u.x, q0, O0.x); O0.y = fma(u.y, q0, O0.y);
-        O1.x = fma(u.x, q1, O1.x); O1.y = fma(u.y, q1, O1.y);
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const double2 u0 = su[r * F + f], u1 = su[(r + 1) * F + f];
+#pragma unroll
+      for (int i = LO; i < NA; ++i) {
+        E[f][i].x = fma(u0.x, qa[i], E[f][i].x);
+        E[f][i].y = fma(u0.y, qa[i], E[f][i].y);
+        O[f][i].x = fma(u1.x, qb[i], O[f][i].x);
+        O[f][i].y = fma(u1.y, qb[i], O[f][i].y);
       }
-      if (r < rend) {  // odd-length tail: one more even degree
-        const double2 u = Uc[r];
-        const double b = bes[r];
-        const double q0 = fma(x0, qb0, b * qa0), q1 = fma(x1, qb1, b * qa1);
-        E0.x = fma(u.x, q0, E0.x); E0.y = fma(u.y, q0, E0.y);
-        E1.x = fma(u.x, q1, E1.x); E1.y = fma(u.y, q1, E1.y);
-      }
-    }
-    if (ok0) {
-      Ef[(size_t)m * P.nh + j0] = E0;
-      Of[(size_t)m * P.nh + j0] = O0;
-    }
-    if (ok1) {
-      Ef[(size_t)m * P.nh + j1] = E1;
-      Of[(size_t)m * P.nh + j1] = O1;
     }
   }
+}
+
+// Item of a block: order, latitude tile, and its significant segments as two bit masks over the
+// order's segments (all latitude groups of the tile; only the upper half of them).  Warp w takes
+// every fourth segment of the union from the w-th on.
+template <int NA, int F>
+__device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const double2* const (&Uf)[F], int f0,
+                                          bool dense, double* sm) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = item.x, hb = item.y;
+  double2* su = reinterpret_cast<double2*>(sm) + (size_t)w * SEG * F;                          // [SEG][F]
+  double* sb = sm + (size_t)SYN_WARPS * SEG * F * 2 + (size_t)w * SEG;                         // [SEG]
+  double2* part = reinterpret_cast<double2*>(sm + (size_t)SYN_WARPS * SEG * (2 * F + 1));      // partial sums
+  const int j0 = 32 * NA * hb + lane;
+  const long long moff = (long long)m * P.nm - (long long)m * (m - 1) / 2;
+  const int seg0 = P.segoff[m];
+  double2 E[F][NA], O[F][NA];
+#pragma unroll
+  for (int f = 0; f < F; ++f)
+#pragma unroll
+    for (int i = 0; i < NA; ++i) E[f][i] = O[f][i] = make_double2(0.0, 0.0);
+  uint32_t left = (uint32_t)(item.z | item.w);
+  for (int n = 0; left; ++n, left &= left - 1) {
+    if ((n & (SYN_WARPS - 1)) != w) continue;
+    const int k = __ffs(left) - 1, s = seg0 + k, l0 = m + SEG * k;
+    const int len = min(SEG, P.lmax + 1 - l0);
+    const long long base = moff + SEG * k;
+    __syncwarp();
+    for (int t = lane; t < SEG; t += 32) {
+      const bool in = t < len;
+      const double c = in ? __dmul_rn(P.cf[base + t], SQRT2_LEGACY) : 0.0;
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        double2 u = make_double2(0.0, 0.0);
+        if (in) u = Uf[f][dense ? (size_t)(l0 + t) * P.nm + m : (size_t)base + t];
+        su[t * F + f] = make_double2(__dmul_rn(u.x, c), __dmul_rn(u.y, c));
+      }
+      sb[t] = in ? P.be[base + t] : 0.0;
+    }
+    __syncwarp();
+    if (NA > 1 && !(((uint32_t)item.z >> k) & 1u)) syn_segment<NA, NA / 2, F>(P, s, j0, len, su, sb, E, O);
+    else syn_segment<NA, 0, F>(P, s, j0, len, su, sb, E, O);
+  }
+  // partial sums [warp][field][latitude group][E | O][lane]
+  constexpr int PER = F * NA * 2;
+#pragma unroll
+  for (int f = 0; f < F; ++f)
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      part[((size_t)w * PER + (f * NA + i) * 2 + 0) * 32 + lane] = E[f][i];
+      part[((size_t)w * PER + (f * NA + i) * 2 + 1) * 32 + lane] = O[f][i];
+    }
+  __syncthreads();
+  for (int q = w; q < F * NA; q += SYN_WARPS) {
+    const int i = q % NA, j = j0 + 32 * i;
+    if (j >= P.nh) continue;
+    double2 e = part[(size_t)(q * 2) * 32 + lane], o = part[(size_t)(q * 2 + 1) * 32 + lane];
+#pragma unroll
+    for (int k = 1; k < SYN_WARPS; ++k) {
+      const double2 e1 = part[((size_t)k * PER + q * 2) * 32 + lane], o1 = part[((size_t)k * PER + q * 2 + 1) * 32 + lane];
+      e = make_double2(__dadd_rn(e.x, e1.x), __dadd_rn(e.y, e1.y));
+      o = make_double2(__dadd_rn(o.x, o1.x), __dadd_rn(o.y, o1.y));
+    }
+    const int f = q / NA;
+    double2* dst = P.EO + (((size_t)(f0 + f) * P.nh + j) * P.nm + m) * 2;
+    dst[0] = e;
+    dst[1] = o;
+  }
+}
+
+constexpr size_t syn_smem(int na, int f) {
+  return (size_t)SYN_WARPS * (SEG * (2 * f + 1) * sizeof(double) + (size_t)f * na * 2 * 32 * sizeof(double2));
+}
+
+// blockIdx.x: the item (most work first); blockIdx.y: the field or the pair of fields, as in the
+// analysis.
+template <int NA, int F>
+__global__ void __launch_bounds__(32 * SYN_WARPS, F == 1 ? 4 : 3) k_leg_syn(sle::ShtDev P, CSpecPtrs in, int nf, int dense) {
+  extern __shared__ double smd[];
+  const int4 item = P.syn_items[blockIdx.x];
+  pdl_wait();
+  pdl_trigger();
+  const int f0 = F * blockIdx.y;
+  int first = -1, count = 0;
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    if (f0 + f < nf && !field_gated_off(P, f0 + f)) {
+      if (first < 0) first = f;
+      ++count;
+    }
+  }
+  if (count == 0) return;
+  if constexpr (F == 2) {
+    if (count == 2) {
+      const double2* const U[2] = {in.p[f0], in.p[f0 + 1]};
+      syn_block<NA, 2>(P, item, U, f0, dense != 0, smd);
+      return;
+    }
+  }
+  const double2* const U[1] = {in.p[f0 + first]};
+  syn_block<NA, 1>(P, item, U, f0 + first, dense != 0, smd);
 }
 
 // ---------------------------------------------------------------- dense <-> packed
@@ -562,10 +668,38 @@ __global__ void k_unpack(sle::ShtDev P, const double2* packed, double2* dense) {
 
 // ------------------------------------------------------------------------ launchers
 static size_t fft_smem(const ShtDev& d) { return fft_smem_bytes(2, d.n2, sizeof(double2)); }
-static int syn_threads(const ShtDev& d) { return 32 * ((d.ngrp + 1) / 2); }
-static size_t syn_smem(const ShtDev& d) { return (size_t)3 * d.nm * sizeof(double); }
+// Latitude groups per lane of the synthesis (and per block): four from three groups on.
+static int syn_na(const ShtDev& d) { return d.ngrp >= 3 ? 4 : d.ngrp; }
+// Whether the Legendre kernels take the fields in pairs (one recurrence for two fields): once the
+// single-field form has more warps than are resident at once (16 per SM) a pair saves work; below
+// that it would only leave schedulers without a warp.  Measured: at L = 255 (640 segments),
+// three fields, 20.0 us single against 22.8 us paired; at L = 63, two fields, 6.6 against 8.7 us; from
+// L = 511 on every number of fields pairs (two fields 42 us, against twice 26 to 28 us for single ones).
+static bool leg_pairs(const sle_sht* plan, int nf) {
+  return nf >= 2 && (long long)plan->d.nseg * nf > 16LL * plan->n_sm;
+}
 
-// One FP64 launch group (1..MAXF fields).
+// The Legendre analysis of nf fields (folded FFTs in d.X).
+static int fp64_leg_ana(const sle_sht* plan, const ShtDev& d, const SpecPtrs& o, int nf, int dense, cudaStream_t st) {
+  const unsigned gx = (unsigned)((d.nseg + ANA_WARPS - 1) / ANA_WARPS);
+  if (leg_pairs(plan, nf))
+    SLE_CUDA(launch_pdl(k_leg_ana<2>, dim3(gx, (nf + 1) / 2), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
+  else
+    SLE_CUDA(launch_pdl(k_leg_ana<1>, dim3(gx, nf), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
+  return SLE_OK;
+}
+
+template <int NA>
+static int fp64_leg_syn(const sle_sht* plan, const ShtDev& d, const CSpecPtrs& c, int nf, int dense, cudaStream_t st) {
+  const unsigned gx = (unsigned)(d.nm * ((d.ngrp + NA - 1) / NA));
+  if (leg_pairs(plan, nf))
+    SLE_CUDA(launch_pdl(k_leg_syn<NA, 2>, dim3(gx, (nf + 1) / 2), dim3(32 * SYN_WARPS), syn_smem(NA, 2), st, d, c, nf, dense));
+  else
+    SLE_CUDA(launch_pdl(k_leg_syn<NA, 1>, dim3(gx, nf), dim3(32 * SYN_WARPS), syn_smem(NA, 1), st, d, c, nf, dense));
+  return SLE_OK;
+}
+
+// One FP64 launch group (1..MAXF fields, all packed or all dense).
 static int fp64_analysis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream_t st, int prof_cls) {
   ShtDev d = plan->d;
   GridPtrs g{};
@@ -580,14 +714,13 @@ static int fp64_analysis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream_
     d.gclr[f] = fs[f].skip_clear;
   }
   ProfToken t0 = prof_begin(PROF_FFT, nf, st);
-#define SLE_LAUNCH_FOLD(NN) k_fft_fold<NN><<<dim3(d.nh, nf), fft_threads(2, NN), fft_smem(d), st>>>(d, g)
+#define SLE_LAUNCH_FOLD(NN) \
+  SLE_CUDA(launch_pdl(k_fft_fold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_FOLD)
 #undef SLE_LAUNCH_FOLD
   prof_end(t0, st);
-  const int warps_per_block = ANA_WARPS;
-  dim3 grid((d.nseg + warps_per_block - 1) / warps_per_block, nf);
   ProfToken t1 = prof_begin(prof_cls, nf, st);
-  k_leg_ana<<<grid, 32 * warps_per_block, 0, st>>>(d, o);
+  SLE_TRY(fp64_leg_ana(plan, d, o, nf, fs[0].dense, st));
   prof_end(t1, st);
   note_launch(2);
   SLE_CUDA(cudaGetLastError());
@@ -606,12 +739,15 @@ static int fp64_synthesis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream
     d.gset[f] = fs[f].skip_set;
     d.gclr[f] = fs[f].skip_clear;
   }
-  const int npairs = (d.nm + 1) / 2;
   ProfToken t0 = prof_begin(PROF_LEG_SYN, nf, st);
-  k_leg_syn<<<dim3(npairs, nf), syn_threads(d), syn_smem(d), st>>>(d, c);
+  const int na = syn_na(d), dense = fs[0].dense;
+  if (na == 4) SLE_TRY(fp64_leg_syn<4>(plan, d, c, nf, dense, st));
+  else if (na == 2) SLE_TRY(fp64_leg_syn<2>(plan, d, c, nf, dense, st));
+  else SLE_TRY(fp64_leg_syn<1>(plan, d, c, nf, dense, st));
   prof_end(t0, st);
   ProfToken t1 = prof_begin(PROF_IFFT, nf, st);
-#define SLE_LAUNCH_IFFT(NN) k_ifft_unfold<NN><<<dim3(d.nh, nf), fft_threads(2, NN), fft_smem(d), st>>>(d, g)
+#define SLE_LAUNCH_IFFT(NN) \
+  SLE_CUDA(launch_pdl(k_ifft_unfold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_IFFT)
 #undef SLE_LAUNCH_IFFT
   prof_end(t1, st);
@@ -701,7 +837,7 @@ static int dalloc(T** p, size_t n) {
 static void plan_free(sle_sht* p) {
   if (!p) return;
   void* ptrs[] = {p->mu, p->w, p->wn, p->ws, p->be, p->cf, p->moff, p->lidx, p->segoff,
-                  p->seg_m, p->seg_l0, p->ana_order, p->seeds, p->tw, p->X, p->EO, p->istart,
+                  p->seg_m, p->seg_l0, p->ana_items, p->syn_items, p->seeds, p->tw, p->X, p->EO, p->istart,
                   p->packbuf, p->mx_xf, p->mx_twf, p->mx_gns, p->mx_bsyn, p->mx_s0, p->mx_abort,
                   p->mx_ana_units, p->mx_syn_units, p->mx_syn_seg, p->mx_tab_ana, p->mx_tab_syn,
                   p->mx_ana_cta, p->mx_syn_cta, p->mx_bpos};
@@ -722,6 +858,12 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   while ((1 << d.log2n2) < d.n2) ++d.log2n2;
   d.ngrp = (d.nh + 31) / 32;
   d.ncoef = (long long)d.nm * (d.nm + 1) / 2;
+  {
+    int dev = 0;
+    SLE_CUDA(cudaGetDevice(&dev));
+    SLE_CUDA(cudaDeviceGetAttribute(&p->n_sm, cudaDevAttrMultiProcessorCount, dev));
+    p->n_sm = std::max(1, p->n_sm);
+  }
   // host tables: packed offsets, segments
   std::vector<long long> moff(d.nm + 1);
   std::vector<int> segoff(d.nm + 1), seg_m, seg_l0;
@@ -745,7 +887,7 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   SLE_TRY(dalloc(&p->segoff, d.nm + 1));
   SLE_TRY(dalloc(&p->seg_m, d.nseg));
   SLE_TRY(dalloc(&p->seg_l0, d.nseg));
-  SLE_TRY(dalloc(&p->ana_order, d.nseg));
+  SLE_TRY(dalloc(&p->ana_items, d.nseg));
   SLE_TRY(dalloc(&p->seeds, (size_t)d.nseg * d.nh));
   SLE_TRY(dalloc(&p->be, d.ncoef));
   SLE_TRY(dalloc(&p->cf, d.ncoef));
@@ -804,7 +946,7 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   d.be = p->be;
   d.cf = p->cf;
   d.istart = p->istart;
-  d.ana_order = p->ana_order;
+  d.ana_items = p->ana_items;
   d.tw = p->tw;
   d.X = p->X;
   d.EO = p->EO;
@@ -853,7 +995,41 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   }
   p->work_frac = total ? (double)done / (double)total : 1.0;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work[a] > work[b]; });
-  SLE_CUDA(cudaMemcpy(p->ana_order, order.data(), d.nseg * sizeof(int), cudaMemcpyHostToDevice));
+  {
+    std::vector<int4> items(d.nseg);
+    for (int i = 0; i < d.nseg; ++i) items[i] = make_int4(order[i], seg_m[order[i]], seg_l0[order[i]], ist[order[i]]);
+    SLE_CUDA(cudaMemcpy(p->ana_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  }
+  {
+    // synthesis blocks: (order, latitude tile) with the tile's significant segments, most work first
+    const int na = syn_na(d), ntile = (d.ngrp + na - 1) / na;
+    std::vector<int4> items;
+    std::vector<long long> cost;
+    for (int m = 0; m < d.nm; ++m) {
+      for (int t = 0; t < ntile; ++t) {
+        const int glo = na * t, ghi = std::min(glo + na, d.ngrp) - 1;
+        uint32_t full = 0, half = 0;
+        long long c = 0;
+        for (int k = 0; segoff[m] + k < segoff[m + 1]; ++k) {
+          const int g = ist[segoff[m] + k];
+          if (g > ghi) continue;
+          const bool upper = na > 1 && g >= glo + na / 2;
+          (upper ? half : full) |= 1u << k;
+          c += (long long)std::min(SEG, lmax + 1 - seg_l0[segoff[m] + k]) * (upper ? 1 : 2);
+        }
+        items.push_back(make_int4(m, t, (int)full, (int)half));
+        cost.push_back(c);
+      }
+    }
+    std::vector<int> by(items.size());
+    std::iota(by.begin(), by.end(), 0);
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::vector<int4> sorted;
+    for (int i : by) sorted.push_back(items[i]);
+    SLE_TRY(dalloc(&p->syn_items, sorted.size()));
+    SLE_CUDA(cudaMemcpy(p->syn_items, sorted.data(), sorted.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    d.syn_items = p->syn_items;
+  }
 
 #define SLE_ATTR_FFT(NN)                                                                              \
   do {                                                                                                \
@@ -864,7 +1040,6 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   } while (0)
   SLE_FFT_SWITCH(d.n2, SLE_ATTR_FFT)
 #undef SLE_ATTR_FFT
-  SLE_CUDA(cudaFuncSetAttribute(k_leg_syn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)syn_smem(d)));
   SLE_CUDA(cudaDeviceSynchronize());
   return SLE_OK;
 }
@@ -998,20 +1173,19 @@ extern "C" int sle_sht_analysis(sle_sht* plan, int nfields, const double* const*
       return SLE_ERR_BAD_ARG;
     }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  std::vector<double2*> outp(nfields);
-  for (int f = 0; f < nfields; ++f)
-    outp[f] = (layout == SLE_LAYOUT_PACKED) ? reinterpret_cast<double2*>(coeffs_dev[f])
-                                            : plan->packbuf + (size_t)f * plan->d.ncoef;
+  // dense layout: the FP64 kernels write it themselves, the mixed ones go through the packed staging
+  const bool staged = layout != SLE_LAYOUT_PACKED && plan->precision == SLE_PREC_MIXED;
   std::vector<FieldSpec> fs(nfields, FieldSpec{});
   for (int f = 0; f < nfields; ++f) {
     fs[f].grid = const_cast<double*>(grids_dev[f]);
-    fs[f].spec = outp[f];
+    fs[f].spec = staged ? plan->packbuf + (size_t)f * plan->d.ncoef : reinterpret_cast<double2*>(coeffs_dev[f]);
+    fs[f].dense = layout != SLE_LAYOUT_PACKED && !staged;
   }
   SLE_TRY(sht_analysis_list(plan, fs.data(), nfields, st));
   SLE_TRY(check_abort(plan));
-  if (layout != SLE_LAYOUT_PACKED)
+  if (staged)
     for (int f = 0; f < nfields; ++f)
-      SLE_TRY(sht_unpack(plan, outp[f], reinterpret_cast<double2*>(coeffs_dev[f]), st));
+      SLE_TRY(sht_unpack(plan, fs[f].spec, reinterpret_cast<double2*>(coeffs_dev[f]), st));
   return SLE_OK;
 }
 
@@ -1032,20 +1206,18 @@ extern "C" int sle_sht_synthesis(sle_sht* plan, int nfields, const void* const* 
       return SLE_ERR_BAD_ARG;
     }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  std::vector<const double2*> inp(nfields);
-  for (int f = 0; f < nfields; ++f) {
-    if (layout == SLE_LAYOUT_PACKED) {
-      inp[f] = reinterpret_cast<const double2*>(coeffs_dev[f]);
-    } else {
-      double2* pb = plan->packbuf + (size_t)f * plan->d.ncoef;
-      SLE_TRY(sht_pack(plan, reinterpret_cast<const double2*>(coeffs_dev[f]), pb, st));
-      inp[f] = pb;
-    }
-  }
+  // dense layout: the FP64 kernels read it themselves, the mixed ones go through the packed staging
+  const bool staged = layout != SLE_LAYOUT_PACKED && plan->precision == SLE_PREC_MIXED;
   std::vector<FieldSpec> fs(nfields, FieldSpec{});
   for (int f = 0; f < nfields; ++f) {
+    double2* in = reinterpret_cast<double2*>(const_cast<void*>(coeffs_dev[f]));
     fs[f].grid = grids_dev[f];
-    fs[f].spec = const_cast<double2*>(inp[f]);
+    fs[f].spec = in;
+    if (staged) {
+      fs[f].spec = plan->packbuf + (size_t)f * plan->d.ncoef;
+      SLE_TRY(sht_pack(plan, in, fs[f].spec, st));
+    }
+    fs[f].dense = layout != SLE_LAYOUT_PACKED && !staged;
   }
   SLE_TRY(sht_synthesis_list(plan, fs.data(), nfields, st));
   return check_abort(plan);
@@ -1156,10 +1328,11 @@ extern "C" int sle_sht_analysis_noalloc(sle_sht* plan, const double* grid_dev, v
   g.p[0] = grid_dev;
   SpecPtrs o{};
   o.p[0] = reinterpret_cast<double2*>(coeffs_packed_dev);
-#define SLE_LAUNCH_FOLD1(NN) k_fft_fold<NN><<<dim3(d.nh, 1), fft_threads(2, NN), fft_smem(d), st>>>(d, g)
+#define SLE_LAUNCH_FOLD1(NN) \
+  SLE_CUDA(launch_pdl(k_fft_fold<NN>, dim3(d.nh, 1), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_FOLD1)
 #undef SLE_LAUNCH_FOLD1
-  k_leg_ana<<<dim3((d.nseg + ANA_WARPS - 1) / ANA_WARPS, 1), 32 * ANA_WARPS, 0, st>>>(d, o);
+  SLE_TRY(fp64_leg_ana(plan, d, o, 1, 0, st));
   SLE_CUDA(cudaGetLastError());
   note_launch(2);
   return SLE_OK;
