@@ -303,6 +303,15 @@ int sle_topo_residual(const double* tp, const double* s, double c, const double*
                       void* scratch, double* out2, void* stream);
 long long sle_topo_scratch_bytes(void);
 
+/* Bisection of that residual, (sum of max(-T0, 0) C0 area - vp) + rhoi / rhow (sum of dI area), over c in
+ * [lo, hi] (init_topo_segmented.py:91-98): `steps` times lo = mid where it is positive, else hi = mid;
+ * *c_out = (lo + hi) / 2.  Arguments as above; scratch of sle_topo_bisect_scratch_bytes() device bytes,
+ * zero before the first call and fit for the next one after each.  Synchronises the stream. */
+int sle_topo_bisect(const double* tp, const double* s, double lo, double hi, int steps, const double* i0,
+                    const double* ip, const unsigned char* gp, const double* wrow, int nlat, int nlon, double rhoi,
+                    double rhow, double vp, void* scratch, double* c_out, void* stream);
+long long sle_topo_bisect_scratch_bytes(void);
+
 /* ------------------------------------------------------- measurement */
 /* Kernel classes timed by sle_prof_*: 0 row FFT + fold, 1 Legendre analysis, 2 Legendre
  * synthesis, 3 inverse FFT + unfold, 4 modal-state advance, 5 the Legendre analysis of the inner

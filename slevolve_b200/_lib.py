@@ -119,6 +119,10 @@ _SIGS = {
                                   C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_double, C.c_void_p,
                                   C.c_void_p, C.c_void_p]),
     "sle_topo_scratch_bytes": (C.c_longlong, []),
+    "sle_topo_bisect": (C.c_int, [C.c_void_p, C.c_void_p, C.c_double, C.c_double, C.c_int, C.c_void_p, C.c_void_p,
+                                  C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_double, C.c_double,
+                                  C.c_void_p, C.POINTER(C.c_double), C.c_void_p]),
+    "sle_topo_bisect_scratch_bytes": (C.c_longlong, []),
     "sle_batch_get": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int]),
     "sle_batch_stream": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "sle_batch_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int),

@@ -84,6 +84,124 @@ __global__ void __launch_bounds__(TOPO_THREADS) k_topo_residual(const double* __
   }
 }
 
+// Bisection of the residual above over c (init_topo_segmented.py:91-98: lo = mid where the residual is
+// positive, else hi = mid) without the host in between.  One launch decides BIS_LEVELS steps: the
+// midpoints of the next steps form a binary tree whose 2^BIS_LEVELS - 1 nodes follow from (lo, hi)
+// alone, so every block sums the two terms for all of them in one read of the grids (33 bytes a
+// cell), and the last block to finish walks the tree.  Bound: latency (launch, one pass over grids
+// that stay in L2, the last block); four levels cost 15 evaluations a cell, about 6 FP64
+// operations each, which hides behind the pass.  The form before, one residual per launch with a
+// host round trip and one thread adding 592 partial sums, took about 60 us a step; a launch here
+// takes about 13 us for four steps (256 x 512; the whole guess of thirteen states 42 -> 20 ms).
+constexpr int BIS_LEVELS = 4;
+constexpr int BIS_NODES = (1 << BIS_LEVELS) - 1;
+constexpr int BIS_BLOCKS = 296;
+
+struct BisState {
+  double lo, hi;
+};
+
+__global__ void __launch_bounds__(TOPO_THREADS) k_topo_bisect(
+    const double* __restrict__ tp, const double* __restrict__ s, double lo0, double hi0, int first, int levels,
+    const double* __restrict__ i0, const double* __restrict__ ip, const unsigned char* __restrict__ gp,
+    const double* __restrict__ wrow, int nlon, long long n, double rhoi, double rhow, double vp, double* partial,
+    BisState* state, unsigned int* counter) {
+  __shared__ double mids[BIS_NODES + 1], sums[TOPO_THREADS / 32][2 * BIS_NODES], res[BIS_NODES + 1];
+  __shared__ bool last;
+  pdl_wait();
+  pdl_trigger();
+  const double lo = first ? lo0 : state->lo, hi = first ? hi0 : state->hi;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x >= 1 && threadIdx.x <= BIS_NODES) {
+    // node i of the tree (1 = the next midpoint, children 2 i: the residual was not positive, hi = mid;
+    // 2 i + 1: it was, lo = mid)
+    const int i = threadIdx.x;
+    double a = lo, b = hi, mid = __dmul_rn(0.5, __dadd_rn(lo, hi));
+    for (int d = 30 - __clz(i); d >= 0; --d) {
+      if ((i >> d) & 1) a = mid;
+      else b = mid;
+      mid = __dmul_rn(0.5, __dadd_rn(a, b));
+    }
+    mids[i] = mid;
+  }
+  __syncthreads();
+  double v[BIS_NODES], d[BIS_NODES];
+#pragma unroll
+  for (int i = 0; i < BIS_NODES; ++i) v[i] = d[i] = 0.0;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    const double t = tp[q], sq = s[q], I0 = i0[q], area = wrow[q / nlon];
+    const double off = __dmul_rn(ip[q], gp[q] ? 1.0 : 0.0);
+    const double rI = __dmul_rn(rhoi, I0);
+    // dI area with the cell grounded at this T0 and without
+    const double dg = __dmul_rn(__dsub_rn(I0, off), area), df = __dmul_rn(__dsub_rn(__dmul_rn(I0, 0.0), off), area);
+#pragma unroll
+    for (int i = 0; i < BIS_NODES; ++i) {
+      const double T0 = __dadd_rn(__dadd_rn(t, mids[i + 1]), sq);
+      const bool g0 = (I0 > 0.0) && ((T0 > 0.0) || (rI > __dmul_rn(rhow, fabs(T0))));
+      const double vol = (T0 < 0.0 && !g0) ? __dmul_rn(-T0, area) : 0.0;
+      v[i] = __dadd_rn(v[i], vol);
+      d[i] = __dadd_rn(d[i], g0 ? dg : df);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < BIS_NODES; ++i) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v[i] = __dadd_rn(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
+      d[i] = __dadd_rn(d[i], __shfl_xor_sync(0xffffffffu, d[i], o));
+    }
+    if (lane == 0) {
+      sums[w][2 * i] = v[i];
+      sums[w][2 * i + 1] = d[i];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * BIS_NODES) {
+    double t = sums[0][threadIdx.x];
+#pragma unroll
+    for (int k = 1; k < TOPO_THREADS / 32; ++k) t = __dadd_rn(t, sums[k][threadIdx.x]);
+    partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int i = w; i < BIS_NODES; i += TOPO_THREADS / 32) {   // a warp per node, fixed order
+    const volatile double* pv = partial + (size_t)(2 * i) * gridDim.x;
+    const volatile double* pd = pv + gridDim.x;
+    double a = 0.0, b = 0.0;
+    for (unsigned int k = lane; k < gridDim.x; k += 32) {
+      a = __dadd_rn(a, pv[k]);
+      b = __dadd_rn(b, pd[k]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a = __dadd_rn(a, __shfl_xor_sync(0xffffffffu, a, o));
+      b = __dadd_rn(b, __shfl_xor_sync(0xffffffffu, b, o));
+    }
+    if (lane == 0) res[i + 1] = __dadd_rn(__dsub_rn(a, vp), __dmul_rn(__ddiv_rn(rhoi, rhow), b));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double a = lo, b = hi;
+    int i = 1;
+    for (int k = 0; k < levels; ++k) {
+      if (res[i] > 0.0) {
+        a = mids[i];
+        i = 2 * i + 1;
+      } else {
+        b = mids[i];
+        i = 2 * i;
+      }
+    }
+    state->lo = a;
+    state->hi = b;
+    *counter = 0u;   // ready for the next launch (stream order)
+  }
+}
+
 }  // namespace
 }  // namespace sle
 
@@ -129,4 +247,34 @@ extern "C" int sle_topo_residual(const double* tp, const double* s, double c, co
 
 extern "C" long long sle_topo_scratch_bytes(void) {
   return (long long)((2 * TOPO_BLOCKS + 2) * sizeof(double) + 16);
+}
+
+extern "C" long long sle_topo_bisect_scratch_bytes(void) {
+  return (long long)(2 * BIS_NODES * BIS_BLOCKS * sizeof(double) + sizeof(BisState) + 16);
+}
+
+extern "C" int sle_topo_bisect(const double* tp, const double* s, double lo, double hi, int steps, const double* i0,
+                               const double* ip, const unsigned char* gp, const double* wrow, int nlat, int nlon,
+                               double rhoi, double rhow, double vp, void* scratch, double* c_out, void* stream) {
+  if (nlat <= 0 || nlon <= 0 || steps < 1 || !tp || !s || !i0 || !ip || !gp || !wrow || !scratch || !c_out) {
+    set_error("sle_topo_bisect: NULL buffer, empty grid or no steps");
+    return SLE_ERR_BAD_ARG;
+  }
+  const long long n = (long long)nlat * nlon;
+  double* part = static_cast<double*>(scratch);
+  BisState* state = reinterpret_cast<BisState*>(part + 2 * BIS_NODES * BIS_BLOCKS);
+  unsigned int* counter = reinterpret_cast<unsigned int*>(state + 1);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const unsigned grid = (unsigned)std::min<long long>((n + TOPO_THREADS - 1) / TOPO_THREADS, BIS_BLOCKS);
+  for (int k = 0; k < steps; k += BIS_LEVELS) {
+    note_launch();
+    SLE_CUDA(launch_pdl(k_topo_bisect, dim3(grid), dim3(TOPO_THREADS), 0, st, tp, s, lo, hi, k == 0 ? 1 : 0,
+                        std::min(BIS_LEVELS, steps - k), i0, ip, gp, wrow, nlon, n, rhoi, rhow, vp, part, state,
+                        counter));
+  }
+  BisState h;
+  SLE_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SLE_CUDA(cudaStreamSynchronize(st));
+  *c_out = 0.5 * (h.lo + h.hi);
+  return SLE_OK;
 }

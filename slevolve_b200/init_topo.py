@@ -101,6 +101,7 @@ class _Grids:
         self.Vp = float(((-Tp).clamp(min=0) * self.Cp * self.area).sum())
         self.scratch = torch.zeros(int(_lib.lib().sle_topo_scratch_bytes()), dtype=torch.uint8, device="cuda")
         self.out2 = (C.c_double * 2)()
+        self.bisect_scratch = None
 
     def grounded(self, I, T):
         return (I > 0) & ((T > 0) | (self.rhoi * I > self.rhow * T.abs()))
@@ -123,14 +124,20 @@ class _Grids:
         return self.out2[0] - self.Vp + self.rhoi / self.rhow * self.out2[1]
 
     def solve_c(self, S, c, half):
-        lo, hi = c - half, c + half
-        for _ in range(60):
-            mid = 0.5 * (lo + hi)
-            if self.residual(S, mid) > 0:
-                lo = mid
-            else:
-                hi = mid
-        return 0.5 * (lo + hi)
+        """60 bisection steps of the residual over c +- half (init_topo_segmented.py:91-98), decided on
+        the device."""
+        nl, no = self.Tp.shape
+        if self.bisect_scratch is None:
+            n = int(_lib.lib().sle_topo_bisect_scratch_bytes())
+            self.bisect_scratch = self.t.zeros(n, dtype=self.t.uint8, device="cuda")
+        out = C.c_double()
+        st = self.t.cuda.current_stream().cuda_stream
+        _lib.check(_lib.lib().sle_topo_bisect(
+            C.c_void_p(self.Tp.data_ptr()), C.c_void_p(S.data_ptr()), float(c - half), float(c + half), 60,
+            C.c_void_p(self.I0.data_ptr()), C.c_void_p(self.Ip.data_ptr()), C.c_void_p(self.gp_u8.data_ptr()),
+            C.c_void_p(self.wrow.data_ptr()), nl, no, self.rhoi, self.rhow, self.Vp,
+            C.c_void_p(self.bisect_scratch.data_ptr()), C.byref(out), C.c_void_p(st)), "sle_topo_bisect")
+        return out.value
 
     def rms(self, f):
         return float(self.t.sqrt((self.area * f * f).sum() / self.area_sum))
