@@ -80,10 +80,9 @@ constexpr int NPAIR = 2;                      // accumulator pairs (chunk k into
 constexpr int BBLOCK = MX_NMAX * KC;          // floats of one synthesis B block
 constexpr int MAX_CTA_UNITS = 16;            // work units per CTA staged in shared memory
 // fixed cost of a work unit (its epilogue), in half-chunk times, from per-CTA timings at L = 511
-// with 32 fields: analysis ~1180 cycles per half + ~5800 per unit, synthesis ~570 per half +
-// ~13800 per unit (measured before its epilogue wrote one 16-byte store per sum pair; its CTAs
-// stay within 3 % of each other)
-constexpr double ANA_UNIT_COST = 5.0;
+// with 32 fields: analysis ~1230 cycles per half + ~3860 per unit, synthesis ~510 per half +
+// ~12600 per unit
+constexpr double ANA_UNIT_COST = 3.0;
 constexpr double SYN_UNIT_COST = 24.0;
 constexpr int NCOLS = MX_NMAX;                // accumulator columns of every launch (2 per field slot)
 static_assert(512 + 16 * MAX_CTA_UNITS <= MISC_BYTES, "misc shared memory too small");
@@ -321,11 +320,11 @@ __device__ __forceinline__ Smem smem_layout(uint8_t* raw, int nst) {
 enum { BAR_FULL = 0, BAR_EMPTY = NSTAGE_MAX, BAR_RAW = 2 * NSTAGE_MAX, BAR_ACCUM = 3 * NSTAGE_MAX,
        BAR_TFREE = 3 * NSTAGE_MAX + 2, BAR_DRAIN = 3 * NSTAGE_MAX + 4, NBAR = 3 * NSTAGE_MAX + 5 };
 static_assert(NBAR * 8 <= 192, "barrier area too small");
+static_assert(MX_MAXF == 32, "the launch's active fields are one 32-bit mask");
 struct Misc {
   uint64_t* bar;
   uint32_t* tmem_holder;
-  int* active;          // [MX_MAXF]
-  int* any;
+  int* any;             // bit f: field f of the launch is active
   int4* units;          // [MAX_CTA_UNITS]: this CTA's work units, staged by the prologue
   __device__ uint32_t b(int i) const { return smem_u32(bar + i); }
 };
@@ -334,8 +333,7 @@ __device__ __forceinline__ Misc misc_layout(const Smem& S) {
   Misc m;
   m.bar = reinterpret_cast<uint64_t*>(p);                      // 17 barriers
   m.tmem_holder = reinterpret_cast<uint32_t*>(p + 192);
-  m.active = reinterpret_cast<int*>(p + 256);
-  m.any = reinterpret_cast<int*>(p + 256 + 4 * MX_MAXF);
+  m.any = reinterpret_cast<int*>(p + 256);
   m.units = reinterpret_cast<int4*>(p + 512);
   return m;
 }
@@ -411,7 +409,11 @@ __device__ uint32_t prologue(const Smem& S, const Misc& M, const MxFieldArgs& a,
     mbar_init(M.b(BAR_DRAIN), 1);
     fence_mbar_init();
   }
-  if (threadIdx.x < MX_MAXF) M.active[threadIdx.x] = (threadIdx.x < a.nf) && !field_off(a, threadIdx.x);
+  if (warp == 0) {   // MX_MAXF = 32: a lane per field
+    const bool on = (int)threadIdx.x < a.nf && !field_off(a, threadIdx.x);
+    const uint32_t act = __ballot_sync(0xffffffffu, on);
+    if (threadIdx.x == 0) *M.any = (int)act;
+  }
   if (warp == W_MMA) {
     tc_alloc(smem_u32(M.tmem_holder), TMEM_COLS);
     tc_relinquish();
@@ -419,14 +421,7 @@ __device__ uint32_t prologue(const Smem& S, const Misc& M, const MxFieldArgs& a,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (threadIdx.x == 0) {
-    int any = 0;
-    for (int f = 0; f < a.nf; ++f) any |= M.active[f];
-    *M.any = any;
-  }
-  const uint32_t t = *M.tmem_holder;
-  __syncthreads();
-  return t;
+  return *M.tmem_holder;
 }
 
 __device__ void epilogue_release(uint32_t tmem) {
@@ -562,11 +557,21 @@ __device__ __forceinline__ void split_b_ana(const Smem& S, int st, int nf, int t
 }
 
 // Synthesis B data of one parity: the raw block lands in the hi tile, already in the tile order,
-// and serves as hi as it is; the lo tile gets TF32(x - trunc(x)).
+// and serves as hi as it is; the lo tile gets TF32(x - trunc(x)).  16-byte vectors; the rows beyond
+// the launch's fields hold whatever the stage held before (their columns are not read).
 __device__ __forceinline__ void split_b_syn(const Smem& S, int st, int nrow, int tid) {
-  const uint32_t* hp = reinterpret_cast<const uint32_t*>(S.b_ptr(st, 0));
-  uint32_t* lp = reinterpret_cast<uint32_t*>(S.b_ptr(st, 1));
-  for (int e = tid; e < nrow * KC; e += 128) lp[e] = lo_of_trunc(__uint_as_float(hp[e]));
+  constexpr int NV = TILE_B / 16 / 128;   // 16-byte vectors per thread of a full tile
+  const uint4* hp = reinterpret_cast<const uint4*>(S.b_ptr(st, 0));
+  uint4* lp = reinterpret_cast<uint4*>(S.b_ptr(st, 1));
+  uint4 v[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    if (128 * q < nrow * (KC / 4)) v[q] = hp[tid + 128 * q];
+#pragma unroll
+  for (int q = 0; q < NV; ++q)
+    if (128 * q < nrow * (KC / 4))
+      lp[tid + 128 * q] = make_uint4(lo_of_trunc(__uint_as_float(v[q].x)), lo_of_trunc(__uint_as_float(v[q].y)),
+                                     lo_of_trunc(__uint_as_float(v[q].z)), lo_of_trunc(__uint_as_float(v[q].w)));
 }
 
 // Work unit u (the CTA's i-th): (m, span | latitude tile, chunk count, first table slot).
@@ -574,6 +579,37 @@ template <bool SYN>
 __device__ __forceinline__ void unit_info(const ShtDev& P, const Misc& M, int u, int i, int4& unit, int& nch) {
   unit = (i < MAX_CTA_UNITS) ? M.units[i] : (SYN ? P.mx_syn_units[u] : P.mx_ana_units[u]);
   nch = SYN ? unit.z : P.ngrp - unit.z;
+}
+
+// Degree 0 in FP64 from the row sums of the fold, U_00 = sqrt(0.5) sum_j S_0(j) / 1.41421356, by the four
+// epilogue warps of the CTA whose run holds the unit (m = 0, span 0), before they wait for its first
+// accumulators: warp w sums the fields w, w + 4, .. (lane-strided partial sums, then a fixed
+// butterfly: the same order in every launch), four fields' loads in flight.
+__device__ __forceinline__ void degree0(const ShtDev& P, const Misc& M, const MxFieldArgs& a, int2 rg, uint32_t act,
+                                        int warp, int lane) {
+  bool mine = false;
+  for (int i = 0; i < rg.y; ++i) {
+    const int4 unit = (i < MAX_CTA_UNITS) ? M.units[i] : P.mx_ana_units[rg.x + i];
+    mine |= unit.x == 0 && unit.y == 0;
+  }
+  if (!mine) return;
+#pragma unroll 1
+  for (int f0 = warp; f0 < a.nf; f0 += 16) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int j = lane; j < P.nh; j += 32) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (f0 + 4 * k < a.nf) acc[k] += P.mx_s0[(size_t)(f0 + 4 * k) * P.nh + j];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int f = f0 + 4 * k;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+      if (lane == 0 && f < a.nf && ((act >> f) & 1u))
+        a.spec[f][0] = make_double2(__dmul_rn(__dsqrt_rn(0.5), acc[k]) / SQRT2_LEGACY, 0.0);
+    }
+  }
 }
 
 // Persistent CTAs (one per SM), each over its own run of work units (P.mx_*_cta).  Analysis
@@ -601,6 +637,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const uint32_t tmem = prologue(S, M, a, SYN ? P.mx_syn_units : P.mx_ana_units, rg, SYN ? 8 : 4);
   if (*M.any && *reinterpret_cast<volatile int*>(P.mx_abort) == 0) {
     const int nrow = 2 * a.nf;
+    const uint32_t act = (uint32_t)*M.any;   // bit f: field f is active
     if (warp == W_LOAD) {
       // ---- loader: half q of the CTA's sequence into stage q % NST
       if (lane == 0) {
@@ -716,12 +753,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int m = unit.x;
         const int j = 128 * unit.y + r;                 // latitude of row r
         const uint32_t rowbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-        const int ncb = (2 * a.nf + 15) / 16;
-        const int cb0 = 2 * h, cb1 = min(ncb, 2 * h + 2);
         float4* gq = reinterpret_cast<float4*>(P.mx_gns) + (size_t)j * P.nm + m;
         const size_t gfield = (size_t)P.nh * P.nm;
         float* ev = S.even() + r;
         bool okp = true;
+#pragma unroll
         for (int par = 0; par < 2; ++par) {
           const bool w = mbar_wait(M.b(BAR_ACCUM + par), (uint32_t)(i & 1), ab);
           if (!__all_sync(0xffffffffu, w)) {
@@ -729,8 +765,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             break;
           }
           tc_fence_after();
-#pragma unroll 1
-          for (int cb = cb0; cb < cb1; ++cb) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int cb = 2 * h + c;
+            const uint32_t on = (act >> (8 * cb)) & 0xffu;   // the block's active fields
+            if (on == 0) continue;
             double v[16];
             if (nch > 0) {
               acc_read(rowbase + PAR_COLS * (uint32_t)par, nch, cb, v);
@@ -742,13 +781,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
               for (int q = 0; q < 16; ++q) ev[(16 * cb + q) * 128] = (float)v[q];
             } else if (j < P.nh) {
+              float4* g0 = gq + (size_t)(8 * cb) * gfield;
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
-                const int f = 8 * cb + q;
-                if (f >= a.nf || !M.active[f]) continue;
                 // the even- and odd-degree sums E, O of latitude j (the unfold forms E +- O)
-                gq[f * gfield] = make_float4(ev[(16 * cb + 2 * q) * 128], ev[(16 * cb + 2 * q + 1) * 128], (float)v[2 * q],
-                                             (float)v[2 * q + 1]);
+                const float4 eo = make_float4(ev[(16 * cb + 2 * q) * 128], ev[(16 * cb + 2 * q + 1) * 128],
+                                              (float)v[2 * q], (float)v[2 * q + 1]);
+                if ((on >> q) & 1u) g0[q * gfield] = eo;
               }
             }
           }
@@ -762,10 +801,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
     } else {
       // ---- analysis epilogue: warps 0-3 (parity 0) and 14-17 (parity 1); warp w owns TMEM lanes
-      // 32 (w mod 4) .. 32 (w mod 4) + 31
+      // 32 (w mod 4) .. 32 (w mod 4) + 31.  The column blocks are unrolled, so that the fields'
+      // pointers are constants of the code, and the active fields are one register mask: with a flag
+      // and a pointer looked up per field and store, the epilogue took longer than the other parity's
+      // MMAs, which waited for it.  With degree 0 moved ahead of the first wait (its CTA finished 15 %
+      // behind the others) the launch went from 88.1 to 78.9 us (32 fields, L = 511; 24.6 to 16.5 at
+      // L = 127).
       const int par = warp >= W_EPI1 ? 1 : 0;
       const int r = 32 * (warp & 3) + lane;
       const double inv = 1.0 / SQRT2_LEGACY;
+      if (par == 0) degree0(P, M, a, rg, act, warp, lane);
+      const int last = act ? (31 - __clz((int)act)) >> 3 : -1;   // the last column block with an active field
       int i = 0;
       for (int u = rg.x; i < rg.y; ++u, ++i) {
         int4 unit;
@@ -774,14 +820,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int m = unit.x;
         const uint32_t lanebase = tmem + PAR_COLS * (uint32_t)par + ((uint32_t)(32 * (warp & 3)) << 16);
         const int le = m + ANA_SPAN * unit.y + 2 * r;   // even degree of row r
-        const int ncb = (2 * a.nf + 15) / 16;
-        // this thread's output element: coefficient (le + par, m) of every field (when le + par <= L)
-        const long long abase = (long long)P.moff[m] + (le - m);
+        // this thread's output element: coefficient (le + par, m) of every field (when le + par <= L;
+        // degree 0 comes from the FP64 row sums)
+        const long long at = (long long)m * P.nm - (long long)m * (m - 1) / 2 + (le - m) + par;
+        const bool live = le + par <= L && at != 0;
         const bool w = mbar_wait(M.b(BAR_ACCUM + par), (uint32_t)(i & 1), ab);
         if (!__all_sync(0xffffffffu, w)) break;
         tc_fence_after();
-        const bool live = le + par <= L;
-        for (int cb = 0; cb < ncb; ++cb) {
+#pragma unroll
+        for (int cb = 0; cb < NCOLS / 16; ++cb) {
+          const uint32_t on = (act >> (8 * cb)) & 0xffu;   // the block's active fields
+          if (on == 0) continue;
           double v[16];
           if (nch > 0) {
             acc_read(lanebase, nch, cb, v);
@@ -789,34 +838,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
             for (int q = 0; q < 16; ++q) v[q] = 0.0;
           }
-          if (cb == ncb - 1) {
+          if (cb == last) {
             // this parity's accumulators are in registers: its TMEM half goes to the next unit
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(M.b(BAR_TFREE + par));
           }
-          if (!live) continue;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int f = 8 * cb + q;
-            if (f >= a.nf || !M.active[f]) continue;
-            a.spec[f][abase + par] = make_double2(v[2 * q] * inv, v[2 * q + 1] * inv);
-          }
-        }
-        if (par == 0 && m == 0 && unit.y == 0) {
-          // degree 0 in FP64 from the row sums of the fold: U_00 = sqrt(0.5) sum_j S_0(j) / 1.41421356;
-          // warp w sums the fields w, w + 4, ... (lane-strided partial sums, then a fixed
-          // butterfly: the same order in every launch)
-          __syncwarp();
-          for (int f = warp; f < a.nf; f += 4) {
-            if (!M.active[f]) continue;
-            const double* s0 = P.mx_s0 + (size_t)f * P.nh;
-            double acc = 0.0;
-            for (int jj = lane; jj < P.nh; jj += 32) acc += s0[jj];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) a.spec[f][0] = make_double2(__dmul_rn(__dsqrt_rn(0.5), acc) / SQRT2_LEGACY, 0.0);
-          }
+          for (int q = 0; q < 8; ++q)
+            if (live && ((on >> q) & 1u)) a.spec[8 * cb + q][at] = make_double2(v[2 * q] * inv, v[2 * q + 1] * inv);
         }
       }
     }
