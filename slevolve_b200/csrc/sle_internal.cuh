@@ -85,7 +85,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 bool pdl_enabled();
 
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t launch_pdl_if(bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                 A&&... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = block;
@@ -95,8 +96,12 @@ inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t sme
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
-  c.numAttrs = pdl_enabled() ? 1 : 0;
+  c.numAttrs = (early && pdl_enabled()) ? 1 : 0;
   return cudaLaunchKernelEx(&c, k, static_cast<A&&>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  return launch_pdl_if(true, k, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 

@@ -409,14 +409,18 @@ __device__ uint32_t prologue(const Smem& S, const Misc& M, const MxFieldArgs& a,
     mbar_init(M.b(BAR_DRAIN), 1);
     fence_mbar_init();
   }
+  if (warp == W_MMA) {
+    tc_alloc(smem_u32(M.tmem_holder), TMEM_COLS);
+    tc_relinquish();
+  }
+  // up to here only the plan's own tables were read; the gates and the operands come from the
+  // kernels before
+  pdl_wait();
+  pdl_trigger();
   if (warp == 0) {   // MX_MAXF = 32: a lane per field
     const bool on = (int)threadIdx.x < a.nf && !field_off(a, threadIdx.x);
     const uint32_t act = __ballot_sync(0xffffffffu, on);
     if (threadIdx.x == 0) *M.any = (int)act;
-  }
-  if (warp == W_MMA) {
-    tc_alloc(smem_u32(M.tmem_holder), TMEM_COLS);
-    tc_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -625,7 +629,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     k_leg_tc(ShtDev P, MxFieldArgs a, int* status, const __grid_constant__ CUtensorMap tmx, int zbox) {
   static_assert(NST % 2 == 0 && NST <= NSTAGE_MAX, "stage count");
   extern __shared__ uint8_t smraw[];
-  pdl_trigger();   // one CTA per SM, all resident: the next kernel may queue behind them
   const Smem S = smem_layout(smraw, NST);
   const Misc M = misc_layout(S);
   const Abort ab{P.mx_abort, status};
@@ -1054,6 +1057,8 @@ __global__ void __launch_bounds__(fft_nt(2, N)) k_unfold_mx(ShtDev P, MxFieldArg
 // tile order (MX_NMAX x 32 per block).  l = 0 is left out (the inverse FFT adds it in FP64);
 // degrees beyond lmax are zero.  Block (segment, group of 4 fields), 64 threads per field.
 __global__ void __launch_bounds__(256) k_bsyn_mx(ShtDev P, MxFieldArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const int s = blockIdx.x;
   const int f = 4 * blockIdx.y + (threadIdx.x >> 6);
   const int t = threadIdx.x & 63;
@@ -1307,6 +1312,13 @@ static int mx_check_args(const MxFieldArgs& a, const char* what) {
   return SLE_OK;
 }
 
+// Whether a tensor-core launch of so many work units may be scheduled while the kernel before it is
+// finishing (programmatic launch; its prologue then overlaps that kernel's tail).  With at most two
+// units per CTA (up to L = 255) the prologue is a tenth of the launch: the 12-member batch step at L =
+// 127 takes 1162 us instead of 1201.  At L = 511 (five to seven units) the 32-member step was 1.2 %
+// slower with it (8117 against 8022 us).
+static bool tc_early(const sle_sht* p, int units) { return units <= 2 * p->n_sm; }
+
 int sht_mx_analysis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t st, int prof_cls) {
   SLE_TRY(sht_mx_prepare(p));
   SLE_TRY(mx_check_args(a, "mixed analysis"));
@@ -1328,9 +1340,11 @@ int sht_mx_analysis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t 
   const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(p->mx_tmap[zi]);
   ProfToken t1 = prof_begin(prof_cls, a.nf, st);
   if (p->tune_stages == 2)
-    k_leg_tc<false, 2><<<p->n_ana_cta, TC_THREADS, mx_smem(2), st>>>(d, a, status, *map, ZBOX[zi]);
+    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_ana_units), k_leg_tc<false, 2>, dim3(p->n_ana_cta), dim3(TC_THREADS),
+                           mx_smem(2), st, d, a, status, *map, ZBOX[zi]));
   else
-    k_leg_tc<false, 4><<<p->n_ana_cta, TC_THREADS, mx_smem(4), st>>>(d, a, status, *map, ZBOX[zi]);
+    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_ana_units), k_leg_tc<false, 4>, dim3(p->n_ana_cta), dim3(TC_THREADS),
+                           mx_smem(4), st, d, a, status, *map, ZBOX[zi]));
   prof_end(t1, st);
   note_launch(2);
   SLE_CUDA(cudaGetLastError());
@@ -1343,11 +1357,13 @@ int sht_mx_synthesis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t
   const ShtDev& d = p->d;
   const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(p->mx_tmap[0]);
   ProfToken t0 = prof_begin(PROF_LEG_SYN, a.nf, st);
-  if (!b_ready) k_bsyn_mx<<<dim3(d.nseg, (a.nf + 3) / 4), 256, 0, st>>>(d, a);
+  if (!b_ready) SLE_CUDA(launch_pdl(k_bsyn_mx, dim3(d.nseg, (a.nf + 3) / 4), dim3(256), 0, st, d, a));
   if (p->tune_stages == 2)
-    k_leg_tc<true, 2><<<p->n_syn_cta, TC_THREADS, mx_smem(2, true), st>>>(d, a, status, *map, 0);
+    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_syn_units), k_leg_tc<true, 2>, dim3(p->n_syn_cta), dim3(TC_THREADS),
+                           mx_smem(2, true), st, d, a, status, *map, 0));
   else
-    k_leg_tc<true, 4><<<p->n_syn_cta, TC_THREADS, mx_smem(4, true), st>>>(d, a, status, *map, 0);
+    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_syn_units), k_leg_tc<true, 4>, dim3(p->n_syn_cta), dim3(TC_THREADS),
+                           mx_smem(4, true), st, d, a, status, *map, 0));
   prof_end(t0, st);
   ProfToken t1 = prof_begin(PROF_IFFT, a.nf, st);
 #define SLE_LAUNCH_MXU(NN) \

@@ -266,6 +266,8 @@ __global__ void k_set_decay(Dev D, int b, double dt) {
 // Step prologue of every slot: stepping slots get their per-step counters reset; the others are
 // marked done (and converged) so that every kernel of the step skips them.
 __global__ void k_step_begin(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= D.nslot) return;
   Scal* sc = D.sc + b;
@@ -352,6 +354,8 @@ __device__ void rot_advance_block(const Dev& D, int b, Scal* sc) {
 // prefetches into L2 the state rows and the load of the block one resident wave further on in
 // launch order, so that the DRAM keeps reading while the blocks before it compute and store.
 __global__ void __launch_bounds__(256) k_advance(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   int bx, by;
   if (threadIdx.x <= D.K && block_ahead(D.adv_ahead, bx, by) && bx > 0 && !D.sc[D.slot0 + by].done) {
     const int b2 = D.slot0 + by;
@@ -408,6 +412,8 @@ __global__ void __launch_bounds__(256) k_advance(Dev D) {
 // beta, C* = C beta (tO = T0 (C* - C*0) is formed by its analysis); at the slot's first step also
 // I* of the previous ice on T0.
 __global__ void k_ice_grid(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (2 * h >= D.ng) return;
@@ -545,6 +551,8 @@ __device__ void rotation_block(const Dev& D, int b, Scal* sc) {
 // previous ice at the slot's first step, else the committed I*_lm of the last step (copied into
 // oldice here).  The last block evaluates the rotation block for the first inner iteration.
 __global__ void k_pre_spec(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   __shared__ double sh[32];
   const SlotStep ss = D.ss[b];
@@ -601,6 +609,8 @@ __global__ void k_pre_spec(Dev D) {
 // that launch's B operand as field b instead of the FP64 spectrum, of which only (0, 0) is kept
 // (the degree-0 term the unfold adds in FP64).
 __global__ void k_b18(Dev D, float* bsyn, const int* bpos) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D.ncoef) return;
@@ -714,6 +724,8 @@ __global__ void k_update(Dev D) {
 
 // sl_tot = sl_inc with conserv added to (0,0) (plain path, solver.py:1017-1021)
 __global__ void k_sltot(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D.ncoef) return;
@@ -872,6 +884,7 @@ __global__ void k_refresh2_x8(Dev D) {
 constexpr int DICE_BLOCKS = 64;
 __global__ void __launch_bounds__(256) k_dice(Dev D) {
   pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   if (sc->converged || !sc->gr_changed) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -889,6 +902,8 @@ __global__ void __launch_bounds__(256) k_dice(Dev D) {
 // The rotation block of the first inner iteration of every stepping slot (one thread per slot),
 // after the step prologue has formed dS_cur and dI.
 __global__ void k_rotation(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   for (int b = threadIdx.x; b < D.nslot; b += blockDim.x) {
     Scal* sc = D.sc + b;
     if (!sc->done && D.tpw) rotation_block(D, b, sc);
@@ -896,6 +911,8 @@ __global__ void k_rotation(Dev D) {
 }
 
 __global__ void k_loop_cond(Dev D, const int* bstatus, cudaGraphConditionalHandle loop) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
@@ -922,6 +939,8 @@ __global__ void k_loop_cond(Dev D, const int* bstatus, cudaGraphConditionalHandl
 
 // After the loop: re-open the slots that step in this call for the post-loop kernels.
 __global__ void k_reopen(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= D.nslot) return;
   if (D.ss[b].active) D.sc[b].done = 0;
@@ -929,6 +948,8 @@ __global__ void k_reopen(Dev D) {
 
 // Radial displacement spectrum (solver.py:1054-1069)
 __global__ void k_rr(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D.ncoef || sc->status) return;
@@ -968,6 +989,8 @@ __global__ void k_rr(Dev D) {
 // and zero at degree 0; each operation rounded as NumPy rounds it.  The degree-2 rotational rates
 // are added on the host.
 __global__ void k_rate_spec(Dev D, double2* rspec, const double* rtab, double* rrec, double* rrot) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const SlotStep& ss = D.ss[b];
   if (!ss.rates || sc->status) return;
@@ -1029,6 +1052,8 @@ __global__ void k_rate_spec(Dev D, double2* rspec, const double* rtab, double* r
 //   Psi = (ttl l^E) A + ttl visc_h,  zero at degree 0;
 // the degree-2 rotational term is added on the host.
 __global__ void k_horiz_spec(Dev D, double2* hspec, const double* htab) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   if (!D.ss[b].horiz || sc->status) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1059,6 +1084,8 @@ __global__ void k_horiz_spec(Dev D, double2* hspec, const double* htab) {
 }
 
 __global__ void k_commit(Dev D, int extrap) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= D.ncoef || sc->status) return;
@@ -1122,6 +1149,8 @@ __global__ void k_commit(Dev D, int extrap) {
 // last block forms U00 = sum_j P~_00 w_j rowsum_j / (nlon 1.41421356), P~_00 = sqrt(0.5).
 // Without diag the three diagnostic grids are written for full analyses instead.
 __global__ void k_post_grid(Dev D, int diag) {
+  pdl_wait();
+  pdl_trigger();
   SLOT_OR_RETURN();
   __shared__ double sh[32];
   const int j = blockIdx.x;
@@ -1189,6 +1218,8 @@ __global__ void k_post_grid(Dev D, int diag) {
 
 // Without the diag option: the (0,0) coefficients of the four diagnostic analyses
 __global__ void k_diag00(Dev D) {
+  pdl_wait();
+  pdl_trigger();
   const int b = D.slot0 + (int)blockIdx.x;
   Scal* sc = D.sc + b;
   if (sc->done || sc->status || threadIdx.x != 0) return;
@@ -1436,7 +1467,8 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   const int nsyn = (int)s->f_syn_sl.size();
   const bool fuse = s->cfg.precision == SLE_PREC_MIXED && s->cfg.opt_dsl && s->plan->mx_ready &&
                     nsyn <= std::min(MX_MAXF, s->plan->tune_fpl);
-  k_b18<<<dim3(nb(nc), B), 256, 0, st>>>(D, fuse ? s->plan->mx_bsyn : nullptr, fuse ? s->plan->mx_bpos : nullptr);
+  SLE_CUDA(launch_pdl(k_b18, dim3(nb(nc), B), dim3(256), 0, st, D, fuse ? s->plan->mx_bsyn : nullptr,
+                      fuse ? s->plan->mx_bpos : nullptr));
   prof_end(t, st);
   SLE_TRY(sht_synthesis_list(s->plan, s->f_syn_sl.data(), nsyn, st, fuse));
   SLE_TRY(sht_analysis_list(s->plan, s->f_ana_ro.data(), (int)s->f_ana_ro.size(), st, PROF_ANA_STEP));
@@ -1446,7 +1478,7 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   prof_end(t, st);
   if (!s->cfg.opt_dsl) {
     note_launch();
-    k_sltot<<<dim3(nb(nc), B), 256, 0, st>>>(D);
+    SLE_CUDA(launch_pdl(k_sltot, dim3(nb(nc), B), dim3(256), 0, st, D));
     SLE_TRY(sht_synthesis_list(s->plan, s->f_syn_sltot.data(), (int)s->f_syn_sltot.size(), st));
   }
   note_launch(2);
@@ -1465,7 +1497,7 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   t = prof_begin(PROF_DICE, act, st);
   SLE_CUDA(launch_pdl(k_dice, dim3(std::min(nb(nc), (unsigned)DICE_BLOCKS), B), dim3(256), 0, st, D));
   prof_end(t, st);
-  k_loop_cond<<<1, 128, 0, st>>>(D, s->bstatus, loop);
+  SLE_CUDA(launch_pdl(k_loop_cond, dim3(1), dim3(128), 0, st, D, s->bstatus, loop));
   SLE_CUDA(cudaGetLastError());
   return SLE_OK;
 }
@@ -1940,13 +1972,13 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
   SLE_CUDA(cudaMemsetAsync(s->bstatus, 0, sizeof(int), st));
   const unsigned UB = (unsigned)B;
   note_launch(3);
-  k_step_begin<<<nb(B, 128), 128, 0, st>>>(D);
+  SLE_CUDA(launch_pdl(k_step_begin, dim3(nb(B, 128)), dim3(128), 0, st, D));
   // ---- modal advance (solver.py:835)
   ProfToken tadv = prof_begin(PROF_ADVANCE, (double)act.size(), st);
-  k_advance<<<dim3(nb(nc) + 1, UB), 256, 0, st>>>(D);
+  SLE_CUDA(launch_pdl(k_advance, dim3(nb(nc) + 1, UB), dim3(256), 0, st, D));
   prof_end(tadv, st);
   // ---- ice and ocean grids, their analyses (the stepping slots only)
-  k_ice_grid<<<dim3(nb(ng / 2), UB), 256, 0, st>>>(D);
+  SLE_CUDA(launch_pdl(k_ice_grid, dim3(nb(ng / 2), UB), dim3(256), 0, st, D));
   SLE_CUDA(cudaGetLastError());
   {
     std::vector<FieldSpec> f;
@@ -1960,8 +1992,8 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
   }
   // ---- first guess
   note_launch(2);
-  k_pre_spec<<<dim3(nb(nc), UB), 256, 0, st>>>(D);
-  k_rotation<<<1, 128, 0, st>>>(D);
+  SLE_CUDA(launch_pdl(k_pre_spec, dim3(nb(nc), UB), dim3(256), 0, st, D));
+  SLE_CUDA(launch_pdl(k_rotation, dim3(1), dim3(128), 0, st, D));
   SLE_CUDA(cudaGetLastError());
 
   // ---- inner fixed-point loop (solver.py:907-1051): a CUDA graph whose WHILE condition is set
@@ -1988,12 +2020,12 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     }
   }
   note_launch();
-  k_reopen<<<nb(B, 128), 128, 0, st>>>(D);
+  SLE_CUDA(launch_pdl(k_reopen, dim3(nb(B, 128)), dim3(128), 0, st, D));
 
   // ---- radial displacement (solver.py:1054-1072)
   if (s->cfg.calcRG) {
     note_launch();
-    k_rr<<<dim3(nb(nc), UB), 256, 0, st>>>(D);
+    SLE_CUDA(launch_pdl(k_rr, dim3(nb(nc), UB), dim3(256), 0, st, D));
     std::vector<FieldSpec> f;
     for (int b : act) f.push_back(fspec(D.g(G_RR, b), D.sp(S_RRLM, b), &s->sc[b].status));
     SLE_TRY(sht_synthesis_list(s->plan, f.data(), (int)f.size(), st));
@@ -2004,21 +2036,22 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     for (int b : act) any_rates |= s->hss[b].rates != 0;
     if (any_rates) {
       note_launch();
-      k_rate_spec<<<dim3(nb(nc), UB), 256, 0, st>>>(D, s->rate_spec, s->rate_tab, s->rate_rec, s->rate_rot);
+      SLE_CUDA(launch_pdl(k_rate_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->rate_spec, s->rate_tab, s->rate_rec,
+                          s->rate_rot));
     }
     bool any_horiz = false;
     for (int b : act) any_horiz |= s->hss[b].horiz != 0;
     if (any_horiz) {
       note_launch();
-      k_horiz_spec<<<dim3(nb(nc), UB), 256, 0, st>>>(D, s->horiz_spec, s->horiz_tab);
+      SLE_CUDA(launch_pdl(k_horiz_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->horiz_spec, s->horiz_tab));
     }
   }
   // ---- commit (solver.py:1080-1096); extrap history (solver_opt.py:817-822)
   note_launch();
-  k_commit<<<dim3(nb(nc), UB), 256, 0, st>>>(D, s->cfg.inner_extrap);
+  SLE_CUDA(launch_pdl(k_commit, dim3(nb(nc), UB), dim3(256), 0, st, D, s->cfg.inner_extrap));
   // ---- topography / ocean function and the degree-0 diagnostics
   note_launch();
-  k_post_grid<<<dim3(D.nlat, UB), 256, 0, st>>>(D, s->cfg.opt_diag);
+  SLE_CUDA(launch_pdl(k_post_grid, dim3(D.nlat, UB), dim3(256), 0, st, D, s->cfg.opt_diag));
   if (!s->cfg.opt_diag) {
     std::vector<FieldSpec> f;
     for (int b : act) {
@@ -2030,7 +2063,7 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     }
     SLE_TRY(sht_analysis_list(s->plan, f.data(), (int)f.size(), st));
     note_launch();
-    k_diag00<<<UB, 32, 0, st>>>(D);
+    SLE_CUDA(launch_pdl(k_diag00, dim3(UB), dim3(32), 0, st, D));
   }
   SLE_CUDA(cudaGetLastError());
   return SLE_OK;
