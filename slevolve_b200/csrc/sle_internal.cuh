@@ -141,6 +141,7 @@ struct ShtDev {
   float* mx_bsyn;             // [nseg][2][MX_NMAX][32] synthesis B operand (FP32, tile order)
   double* mx_s0;              // [MX_MAXF][nh] FP64 fold of the row sums (degree 0)
   int* mx_abort;              // raised by a tensor-core kernel whose wait timed out
+  int* mx_abort_host;         // the same in mapped host memory (device address)
   const int4* mx_ana_units;   // (m, span, first chunk, table slot) analysis units, in runs per CTA
   const int4* mx_syn_units;   // (m, latitude tile, chunks, table slot) synthesis units
   const int2* mx_ana_cta;     // (first unit, units) of each CTA of an analysis launch
@@ -256,6 +257,7 @@ struct sle_sht {
   int* mx_bpos;                  // [ncoef] synthesis B position of each packed coefficient (mx_bsyn_put)
   double* mx_s0;
   int* mx_abort;
+  int* mx_abort_host;            // mapped host memory
   int4 *mx_ana_units, *mx_syn_units;
   int2 *mx_ana_cta, *mx_syn_cta;
   int* mx_syn_seg;
@@ -304,6 +306,6 @@ int sht_mx_analysis(sle_sht* plan, const MxFieldArgs& a, int* status, cudaStream
                     int prof_cls = PROF_LEG_ANA);
 // b_ready: the synthesis B operand of the launch's fields is already in place (mx_bsyn_put)
 int sht_mx_synthesis(sle_sht* plan, const MxFieldArgs& a, int* status, cudaStream_t st, bool b_ready = false);
-int sht_mx_abort_flag(sle_sht* plan, int* flag);
+int sht_mx_abort_flag(sle_sht* plan, int* flag, cudaStream_t st);
 int sht_unpack(sle_sht* plan, const double2* packed, double2* dense, cudaStream_t st);
 }  // namespace sle

@@ -228,11 +228,14 @@ __device__ __forceinline__ uint32_t lo_of_trunc(float x) {
 // ------------------------------------------------------------------ bounded waits
 struct Abort {
   int* flag;     // plan-wide abort word
+  int* host;     // its copy in mapped host memory, which a finished call reads without a copy
   int* status;   // caller's status word (may be null)
 };
 
 __device__ __forceinline__ void raise_abort(const Abort& ab) {
   atomicExch(ab.flag, 1);
+  *reinterpret_cast<volatile int*>(ab.host) = 1;
+  __threadfence_system();
   if (ab.status) atomicExch(ab.status, SLE_ERR_TIMEOUT);
 }
 
@@ -631,7 +634,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   extern __shared__ uint8_t smraw[];
   const Smem S = smem_layout(smraw, NST);
   const Misc M = misc_layout(S);
-  const Abort ab{P.mx_abort, status};
+  const Abort ab{P.mx_abort, P.mx_abort_host, status};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int L = P.lmax;
   const uint32_t* tab = SYN ? P.mx_tab_syn : P.mx_tab_ana;
@@ -1127,6 +1130,9 @@ int sht_mx_prepare(sle_sht* p) {
   SLE_CUDA(cudaMemset(p->mx_gns, 0, 2 * nx4 * sizeof(float2)));
   SLE_CUDA(cudaMemset(p->mx_bsyn, 0, (size_t)d.nseg * 2 * BBLOCK * sizeof(float)));
   SLE_CUDA(cudaMemset(p->mx_abort, 0, sizeof(int)));
+  SLE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p->mx_abort_host), sizeof(int), cudaHostAllocMapped));
+  *p->mx_abort_host = 0;
+  SLE_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&d.mx_abort_host), p->mx_abort_host, 0));
   {
     // FP32 twiddle table (same layout), rounded from the plan's FP64 one
     const int ntw = tw_table_len(d.n2);
@@ -1376,10 +1382,23 @@ int sht_mx_synthesis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t
   return SLE_OK;
 }
 
-int sht_mx_abort_flag(sle_sht* p, int* flag) {
+// The abort flag after the work enqueued on `st`: waits for the stream and reads the host copy (a
+// device-to-host copy of one word costs a transfer more per call).  As with such a copy on the legacy
+// default stream, a non-blocking stream is not waited for: the call returns at once and reports what
+// earlier, finished work raised.  While the stream is being captured the copy stays.
+int sht_mx_abort_flag(sle_sht* p, int* flag, cudaStream_t st) {
   *flag = 0;
   if (!p->mx_ready) return SLE_OK;
-  SLE_CUDA(cudaMemcpy(flag, p->mx_abort, sizeof(int), cudaMemcpyDeviceToHost));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  SLE_CUDA(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) {
+    SLE_CUDA(cudaMemcpy(flag, p->mx_abort, sizeof(int), cudaMemcpyDeviceToHost));
+    return SLE_OK;
+  }
+  unsigned int kind = cudaStreamDefault;
+  if (st) SLE_CUDA(cudaStreamGetFlags(st, &kind));
+  if (!(kind & cudaStreamNonBlocking)) SLE_CUDA(cudaStreamSynchronize(st));
+  *flag = *reinterpret_cast<volatile int*>(p->mx_abort_host);
   return SLE_OK;
 }
 

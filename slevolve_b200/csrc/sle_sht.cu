@@ -843,6 +843,7 @@ static void plan_free(sle_sht* p) {
                   p->mx_ana_cta, p->mx_syn_cta, p->mx_bpos};
   for (void* q : ptrs)
     if (q) cudaFree(q);
+  if (p->mx_abort_host) cudaFreeHost(p->mx_abort_host);
   delete p;
 }
 
@@ -1145,10 +1146,10 @@ static bool aligned16(const void* p) { return p && (reinterpret_cast<uintptr_t>(
 
 // A mixed-precision kernel that timed out leaves the plan's abort flag raised: report it (the
 // check synchronises only on plans that use the tensor-core path).
-static int check_abort(sle_sht* plan) {
+static int check_abort(sle_sht* plan, cudaStream_t st) {
   if (plan->precision != SLE_PREC_MIXED) return SLE_OK;
   int flag = 0;
-  SLE_TRY(sht_mx_abort_flag(plan, &flag));
+  SLE_TRY(sht_mx_abort_flag(plan, &flag, st));
   if (flag) {
     set_error("a tensor-core transform kernel timed out waiting on its pipeline");
     return SLE_ERR_TIMEOUT;
@@ -1182,7 +1183,7 @@ extern "C" int sle_sht_analysis(sle_sht* plan, int nfields, const double* const*
     fs[f].dense = layout != SLE_LAYOUT_PACKED && !staged;
   }
   SLE_TRY(sht_analysis_list(plan, fs.data(), nfields, st));
-  SLE_TRY(check_abort(plan));
+  SLE_TRY(check_abort(plan, st));
   if (staged)
     for (int f = 0; f < nfields; ++f)
       SLE_TRY(sht_unpack(plan, fs[f].spec, reinterpret_cast<double2*>(coeffs_dev[f]), st));
@@ -1220,7 +1221,7 @@ extern "C" int sle_sht_synthesis(sle_sht* plan, int nfields, const void* const* 
     fs[f].dense = layout != SLE_LAYOUT_PACKED && !staged;
   }
   SLE_TRY(sht_synthesis_list(plan, fs.data(), nfields, st));
-  return check_abort(plan);
+  return check_abort(plan, st);
 }
 
 extern "C" int sle_sht_set_precision(sle_sht* plan, int precision) {

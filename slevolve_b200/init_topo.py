@@ -72,25 +72,31 @@ def relaxed_love(love, lmax, tau):
     """Load Love numbers h, k of degrees 0..lmax relaxed for ``tau`` kyr: the elastic values plus
     sum_k r_k / s_k (1 - exp(-s_k tau)) over the degree's modes (init_topo_segmented.py:114-118)."""
     h, k = np.array(love.he[:lmax + 1], float), np.array(love.ke[:lmax + 1], float)
-    for ll in range(1, lmax + 1):
-        nm = int(love.nmod[ll])
-        s = love.s[:nm, ll]
-        f = 1.0 - np.exp(-s * tau)
-        h[ll] += (love.r[:nm, ll] / s * f).sum()
-        k[ll] += (love.rprime[:nm, ll] / s * f).sum()
+    nl = lmax + 1
+    nm = np.asarray(love.nmod[:nl], int)
+    K = int(nm[1:].max()) if nl > 1 else 0
+    if K == 0:
+        return h, k
+    on = np.arange(K)[:, None] < nm[None, :]   # the degree's modes
+    on[:, 0] = False
+    s = np.where(on, love.s[:K, :nl], 1.0)
+    f = np.where(on, (1.0 - np.exp(-s * tau)) / s, 0.0)
+    h += (np.where(on, love.r[:K, :nl], 0.0) * f).sum(axis=0)
+    k += (np.where(on, love.rprime[:K, :nl], 0.0) * f).sum(axis=0)
     return h, k
 
 
 class _Grids:
     """Present state, areas and the conservation residual on the device."""
 
-    def __init__(self, Tp, I0, Ip, rhoi, rhow, radius, torch):
+    def __init__(self, Tp, I0, Ip, rhoi, rhow, radius, torch, weights=None):
         self.t = torch
         self.Tp, self.I0, self.Ip = Tp, I0, Ip
         self.rhoi, self.rhow = float(rhoi), float(rhow)
         nl, no = Tp.shape
-        _, gw = np.polynomial.legendre.leggauss(nl)
-        wrow = gw[::-1] * 2 * np.pi / no * radius ** 2
+        if weights is None:
+            weights = np.polynomial.legendre.leggauss(nl)[1][::-1]
+        wrow = np.asarray(weights, float) * 2 * np.pi / no * radius ** 2
         self.wrow = torch.from_numpy(np.ascontiguousarray(wrow)).cuda()
         self.area = self.wrow[:, None].expand(nl, no).contiguous()
         self.area_sum = self.area.sum()
@@ -162,10 +168,13 @@ def segmented_guess(Tp, ice, love, lmax, dt, threshold=0.01, start=None, c0=62.0
     Tp_d = dev(Tp)
     nl, no = Tp_d.shape
     N = len(ice) - 1
-    g = _Grids(Tp_d, dev(ice[0]), dev(ice[N]), rhoi, rhow, radius, torch)
+    sht = sht if sht is not None else make_sht("cuda", nl, no, lmax)
+    # the transform's own Gauss weights (leggauss solves an eigenvalue problem for them)
+    weights = getattr(sht, "weights", None)
+    g = _Grids(Tp_d, dev(ice[0]), dev(ice[N]), rhoi, rhow, radius, torch,
+               weights if weights is not None and len(weights) == nl else None)
     V = np.array([float((dev(ice[n]) * g.area).sum()) for n in range(N + 1)])
     segs = segments(V, dt, threshold)
-    sht = sht if sht is not None else make_sht("cuda", nl, no, lmax)
     l = np.arange(lmax + 1, dtype=float)
     ttl = np.zeros_like(l)
     ttl[1:] = 4 * np.pi * radius ** 3 / (MASS * (2 * l[1:] + 1))
