@@ -105,6 +105,26 @@ inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t sme
 }
 
 
+// Shared-memory share (percent of 228 KB: the 100 KB setting) that every kernel but the tensor-core ones
+// asks for.  Kernels that ask for different shares cannot share an SM, so that a kernel scheduled early
+// waits for the SM to drain and reconfigure; and the row FFTs read their twiddles through the L1 that
+// the rest leaves (32-field fold at L = 511: 69.4 us at 100 percent, 58.4 at 44, 84.4 at 28, where
+// fewer blocks fit).  FP64 step at L = 511 773 -> 734 us, 32-member batch step 7290 -> 7160 us.
+constexpr int SMEM_CARVEOUT = 44;
+
+// What the FP64 Legendre kernels walk: pieces of fseg degrees (a segment or an even fraction of one),
+// their seeds, the first piece of each order, and the work items.
+struct LegSet {
+  int fseg, nfseg;
+  const double2* fseeds;      // [nfseg][nh], in the segment's scale
+  const int* fsegoff;         // [nm+1]
+  // analysis: (piece, order, first degree, first significant latitude group), most work first;
+  // synthesis: (order, latitude tile, mask of the order's pieces significant on the whole tile, mask
+  // of those significant on its upper half only), most work first
+  const int4* ana_items;      // [nfseg]
+  const int4* syn_items;      // [nm * tiles]
+};
+
 // Device view of a transform plan, passed to kernels by value.
 struct ShtDev {
   int nlat, nlon, lmax, nh, nm, n2, log2n2, ngrp, nseg;
@@ -122,11 +142,7 @@ struct ShtDev {
   const double* be;           // [ncoef] Q_l = mu Q_{l-1} + be_l Q_{l-2}
   const double* cf;           // [ncoef] P~_l = cf_l Q_l (segment scale)
   const unsigned char* istart;// [nseg] first significant latitude group of the segment
-  // FP64 analysis: (segment, order, first degree, first significant latitude group), most work first;
-  // synthesis: (order, latitude tile, mask of the order's segments significant on the whole tile, mask
-  // of those significant on its upper half only), most work first
-  const int4* ana_items;      // [nseg]
-  const int4* syn_items;      // [nm * tiles]
+  LegSet leg;                 // what a launch of the FP64 Legendre kernels walks
   const double2* tw;          // [n2] exp(-2 pi i t / nlon)
   double2* X;                 // [MAXF][2][nm][nh] folded rFFT (S then D) of analysed grids
   double2* EO;                // [MAXF][nh][nm][2] even/odd Legendre sums of synthesised fields
@@ -240,7 +256,7 @@ struct sle_sht {
   double *mu, *w, *wn, *ws, *be, *cf;
   long long* moff;
   int *lidx, *segoff, *seg_m, *seg_l0;
-  int4 *ana_items, *syn_items;
+  sle::LegSet leg[2];         // FP64 Legendre kernels: the segments, and shorter pieces (may be the same)
   double2 *seeds, *tw, *X, *EO;
   unsigned char* istart;
   double2* packbuf;           // [MAXF][ncoef] packed staging for dense-layout calls

@@ -1295,15 +1295,16 @@ int sht_mx_prepare(sle_sht* p) {
 #define SLE_ATTR_MX(NN)                                                                                        \
   do {                                                                                                         \
     SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_fold_smem(d, 4)));    \
-    SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)); \
+    SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT)); \
     SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_fold_smem(d, 8)));    \
-    SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 8>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)); \
+    SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 8>, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT)); \
     SLE_CUDA(cudaFuncSetAttribute(k_unfold_mx<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_unfold_smem(d)));      \
-    SLE_CUDA(cudaFuncSetAttribute(k_unfold_mx<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)); \
+    SLE_CUDA(cudaFuncSetAttribute(k_unfold_mx<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT)); \
     SLE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p->unfold_ahead, k_unfold_mx<NN>,                    \
                                                            fft_threads(2, NN), mx_unfold_smem(d)));              \
   } while (0)
   SLE_FFT_SWITCH(d.n2, SLE_ATTR_MX)
+  SLE_CUDA(cudaFuncSetAttribute(k_bsyn_mx, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT));
 #undef SLE_ATTR_MX
   p->unfold_ahead *= p->n_sm;
   p->mx_ready = 1;

@@ -172,6 +172,25 @@ __global__ void k_istart(sle::ShtDev P, const double* segmax, unsigned char* ist
   istart[s] = (unsigned char)g;
 }
 
+// Seeds of the pieces of fseg degrees that the FP64 kernels walk: the recurrence carried through each
+// segment with the kernels' own operations, its state (Q_{l0-2}, Q_{l0-1}) stored where a piece starts.
+__global__ void k_piece_seeds(sle::ShtDev P, double2* out) {
+  const int s = blockIdx.x, m = P.seg_m[s], l0 = P.seg_l0[s];
+  const int len = min(SEG, P.lmax + 1 - l0), first = P.leg.fsegoff[m] + (l0 - m) / P.leg.fseg;
+  const long long base = P.moff[m] + (l0 - m);
+  for (int j = threadIdx.x; j < P.nh; j += blockDim.x) {
+    const double mu = P.mu[j];
+    const double2 sd = P.seeds[(size_t)s * P.nh + j];
+    double qa = sd.x, qb = sd.y;
+    for (int t = 0; t < len; ++t) {
+      if (t % P.leg.fseg == 0) out[(size_t)(first + t / P.leg.fseg) * P.nh + j] = make_double2(qa, qb);
+      const double q = fma(mu, qb, __dmul_rn(P.be[base + t], qa));
+      qa = qb;
+      qb = q;
+    }
+  }
+}
+
 __global__ void k_lidx(sle::ShtDev P, int* lidx) {
   const int m = blockIdx.x;
   const long long base = P.moff[m];
@@ -351,7 +370,7 @@ __device__ __forceinline__ void ana_pass(const sle::ShtDev& P, int s, int m, int
     const int j = (g0 + i) * 32 + lane;
     const bool ok = j < nh;
     mu[i] = ok ? P.mu[j] : 0.0;
-    const double2 sd = ok ? P.seeds[(size_t)s * nh + j] : make_double2(0.0, 0.0);
+    const double2 sd = ok ? P.leg.fseeds[(size_t)s * nh + j] : make_double2(0.0, 0.0);
     qa[i] = sd.x;
     qb[i] = sd.y;
 #pragma unroll
@@ -412,8 +431,8 @@ __device__ __forceinline__ void ana_segment(const sle::ShtDev& P, int s, int m, 
                                             const double2* const (&Xf)[F], double2* const (&Uf)[F], bool dense,
                                             int lane, const double* __restrict__ sbe, const double* __restrict__ scf,
                                             double* __restrict__ red, double* __restrict__ sacc) {
-  const int len = min(SEG, P.lmax + 1 - l0);
-  const long long base = P.moff[m] + (l0 - m);
+  const int len = min(P.leg.fseg, P.lmax + 1 - l0);
+  const long long base = (long long)m * P.nm - (long long)m * (m - 1) / 2 + (l0 - m);
   bool more = false;
   int g = gs;
   while (g < P.ngrp) {
@@ -454,17 +473,17 @@ __global__ void __launch_bounds__(32 * ANA_WARPS, F == 1 ? 6 : 4) k_leg_ana(sle:
   const int wib = threadIdx.x >> 5;
   const int warp = blockIdx.x * ANA_WARPS + wib;
   const int lane = threadIdx.x & 31;
-  if (warp >= P.nseg) {
+  if (warp >= P.leg.nfseg) {
     pdl_wait();
     return;
   }
-  const int4 item = P.ana_items[warp];   // segment, order, first degree, first significant group
+  const int4 item = P.leg.ana_items[warp];   // segment, order, first degree, first significant group
   double* sbe = scoef[wib][0];
   double* scf = scoef[wib][1];
   {
-    const int len = min(SEG, P.lmax + 1 - item.z);
+    const int len = min(P.leg.fseg, P.lmax + 1 - item.z);
     const long long base = (long long)item.y * P.nm - (long long)item.y * (item.y - 1) / 2 + (item.z - item.y);
-    for (int t = lane; t < SEG; t += 32) {
+    for (int t = lane; t < P.leg.fseg; t += 32) {
       sbe[t] = (t < len) ? P.be[base + t] : 0.0;
       scf[t] = (t < len) ? __ddiv_rn(P.cf[base + t], SQRT2_LEGACY) : 0.0;
     }
@@ -522,7 +541,7 @@ __device__ __forceinline__ void syn_segment(const sle::ShtDev& P, int s, int j0,
     const int j = j0 + 32 * i;
     const bool ok = j < P.nh;
     x[i] = ok ? P.mu[j] : 0.0;
-    const double2 sd = ok ? P.seeds[(size_t)s * P.nh + j] : make_double2(0.0, 0.0);
+    const double2 sd = ok ? P.leg.fseeds[(size_t)s * P.nh + j] : make_double2(0.0, 0.0);
     qa[i] = sd.x;
     qb[i] = sd.y;
   }
@@ -561,7 +580,7 @@ __device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const
   double2* part = reinterpret_cast<double2*>(sm + (size_t)SYN_WARPS * SEG * (2 * F + 1));      // partial sums
   const int j0 = 32 * NA * hb + lane;
   const long long moff = (long long)m * P.nm - (long long)m * (m - 1) / 2;
-  const int seg0 = P.segoff[m];
+  const int seg0 = P.leg.fsegoff[m];
   double2 E[F][NA], O[F][NA];
 #pragma unroll
   for (int f = 0; f < F; ++f)
@@ -570,11 +589,11 @@ __device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const
   uint32_t left = (uint32_t)(item.z | item.w);
   for (int n = 0; left; ++n, left &= left - 1) {
     if ((n & (SYN_WARPS - 1)) != w) continue;
-    const int k = __ffs(left) - 1, s = seg0 + k, l0 = m + SEG * k;
-    const int len = min(SEG, P.lmax + 1 - l0);
-    const long long base = moff + SEG * k;
+    const int k = __ffs(left) - 1, s = seg0 + k, l0 = m + P.leg.fseg * k;
+    const int len = min(P.leg.fseg, P.lmax + 1 - l0);
+    const long long base = moff + P.leg.fseg * k;
     __syncwarp();
-    for (int t = lane; t < SEG; t += 32) {
+    for (int t = lane; t < P.leg.fseg; t += 32) {
       const bool in = t < len;
       const double c = in ? __dmul_rn(P.cf[base + t], SQRT2_LEGACY) : 0.0;
 #pragma unroll
@@ -625,7 +644,7 @@ constexpr size_t syn_smem(int na, int f) {
 template <int NA, int F>
 __global__ void __launch_bounds__(32 * SYN_WARPS, F == 1 ? 4 : 3) k_leg_syn(sle::ShtDev P, CSpecPtrs in, int nf, int dense) {
   extern __shared__ double smd[];
-  const int4 item = P.syn_items[blockIdx.x];
+  const int4 item = P.leg.syn_items[blockIdx.x];
   pdl_wait();
   pdl_trigger();
   const int f0 = F * blockIdx.y;
@@ -679,9 +698,21 @@ static bool leg_pairs(const sle_sht* plan, int nf) {
   return nf >= 2 && (long long)plan->d.nseg * nf > 16LL * plan->n_sm;
 }
 
+// The pieces an analysis of nf fields walks: the short ones while their warps are resident at once (12
+// per SM).  Up to there the kernel waits on its own chains, and shorter ones end earlier; beyond, more
+// pieces only read more seeds.  The sums over the latitudes do not depend on it.  Fold and analysis of
+// one field, segments -> pieces: 6.5 -> 4.5 us at L = 63, 10.5 -> 8.1 at L = 255; three fields at L = 127
+// (2112 pieces) 8.9 -> 11.2, so segments there.  The synthesis, whose sums over the degrees are grouped by
+// piece, takes the plan's short pieces for every number of fields (a field's result does not depend
+// on the others): 4.7 -> 4.0 us at L = 63, 9.3 -> 6.7 for two fields at L = 127.
+static const LegSet& ana_set(const sle_sht* plan, int nf) {
+  return plan->leg[(long long)plan->leg[1].nfseg * nf <= 12LL * plan->n_sm ? 1 : 0];
+}
+
 // The Legendre analysis of nf fields (folded FFTs in d.X).
-static int fp64_leg_ana(const sle_sht* plan, const ShtDev& d, const SpecPtrs& o, int nf, int dense, cudaStream_t st) {
-  const unsigned gx = (unsigned)((d.nseg + ANA_WARPS - 1) / ANA_WARPS);
+static int fp64_leg_ana(const sle_sht* plan, ShtDev d, const SpecPtrs& o, int nf, int dense, cudaStream_t st) {
+  d.leg = ana_set(plan, nf);
+  const unsigned gx = (unsigned)((d.leg.nfseg + ANA_WARPS - 1) / ANA_WARPS);
   if (leg_pairs(plan, nf))
     SLE_CUDA(launch_pdl(k_leg_ana<2>, dim3(gx, (nf + 1) / 2), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
   else
@@ -690,7 +721,8 @@ static int fp64_leg_ana(const sle_sht* plan, const ShtDev& d, const SpecPtrs& o,
 }
 
 template <int NA>
-static int fp64_leg_syn(const sle_sht* plan, const ShtDev& d, const CSpecPtrs& c, int nf, int dense, cudaStream_t st) {
+static int fp64_leg_syn(const sle_sht* plan, ShtDev d, const CSpecPtrs& c, int nf, int dense, cudaStream_t st) {
+  d.leg = plan->leg[1];
   const unsigned gx = (unsigned)(d.nm * ((d.ngrp + NA - 1) / NA));
   if (leg_pairs(plan, nf))
     SLE_CUDA(launch_pdl(k_leg_syn<NA, 2>, dim3(gx, (nf + 1) / 2), dim3(32 * SYN_WARPS), syn_smem(NA, 2), st, d, c, nf, dense));
@@ -834,10 +866,18 @@ static int dalloc(T** p, size_t n) {
   return SLE_OK;
 }
 
+static void leg_set_free(LegSet& a, const double2* segment_seeds) {
+  const void* ptrs[] = {a.fsegoff, a.ana_items, a.syn_items, a.fseeds == segment_seeds ? nullptr : a.fseeds};
+  for (const void* q : ptrs)
+    if (q) cudaFree(const_cast<void*>(q));
+}
+
 static void plan_free(sle_sht* p) {
   if (!p) return;
+  if (p->leg[1].fsegoff != p->leg[0].fsegoff) leg_set_free(p->leg[1], p->seeds);
+  leg_set_free(p->leg[0], p->seeds);
   void* ptrs[] = {p->mu, p->w, p->wn, p->ws, p->be, p->cf, p->moff, p->lidx, p->segoff,
-                  p->seg_m, p->seg_l0, p->ana_items, p->syn_items, p->seeds, p->tw, p->X, p->EO, p->istart,
+                  p->seg_m, p->seg_l0, p->seeds, p->tw, p->X, p->EO, p->istart,
                   p->packbuf, p->mx_xf, p->mx_twf, p->mx_gns, p->mx_bsyn, p->mx_s0, p->mx_abort,
                   p->mx_ana_units, p->mx_syn_units, p->mx_syn_seg, p->mx_tab_ana, p->mx_tab_syn,
                   p->mx_ana_cta, p->mx_syn_cta, p->mx_bpos};
@@ -845,6 +885,81 @@ static void plan_free(sle_sht* p) {
     if (q) cudaFree(q);
   if (p->mx_abort_host) cudaFreeHost(p->mx_abort_host);
   delete p;
+}
+
+// Pieces of SEG / split degrees with their seeds (split 1: the segments' own), and the work items of
+// the FP64 Legendre kernels over them.
+static int leg_set_build(sle_sht* p, LegSet& set, int split, const std::vector<int>& segoff,
+                         const std::vector<unsigned char>& ist) {
+  ShtDev d = p->d;
+  const int L = d.lmax;
+  set = LegSet{};
+  set.fseg = SEG / split;
+  std::vector<int> foff(d.nm + 1), f_m, f_l0, f_ist;
+  for (int m = 0; m < d.nm; ++m) {
+    foff[m] = (int)f_m.size();
+    for (int l0 = m; l0 <= L; l0 += set.fseg) {
+      f_m.push_back(m);
+      f_l0.push_back(l0);
+      f_ist.push_back(ist[segoff[m] + (l0 - m) / SEG]);
+    }
+  }
+  foff[d.nm] = set.nfseg = (int)f_m.size();
+  int* off = nullptr;
+  SLE_TRY(dalloc(&off, d.nm + 1));
+  set.fsegoff = off;
+  SLE_CUDA(cudaMemcpy(off, foff.data(), foff.size() * sizeof(int), cudaMemcpyHostToDevice));
+  set.fseeds = p->seeds;
+  if (split > 1) {
+    double2* seeds = nullptr;
+    SLE_TRY(dalloc(&seeds, (size_t)set.nfseg * d.nh));
+    set.fseeds = seeds;
+    d.leg = set;
+    k_piece_seeds<<<d.nseg, std::min(256, 32 * d.ngrp)>>>(d, seeds);
+    SLE_CUDA(cudaGetLastError());
+  }
+  const auto by_work = [](const std::vector<long long>& work) {   // most work first
+    std::vector<int> order(work.size());
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work[a] > work[b]; });
+    return order;
+  };
+  const auto upload = [](const std::vector<int4>& items, const std::vector<int>& order, const int4** out) -> int {
+    std::vector<int4> v;
+    for (int i : order) v.push_back(items[i]);
+    int4* dev = nullptr;
+    SLE_TRY(dalloc(&dev, v.size()));
+    *out = dev;
+    SLE_CUDA(cudaMemcpy(dev, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    return SLE_OK;
+  };
+  std::vector<int4> items;
+  std::vector<long long> work;
+  for (int i = 0; i < set.nfseg; ++i) {
+    items.push_back(make_int4(i, f_m[i], f_l0[i], f_ist[i]));
+    work.push_back((long long)std::min(set.fseg, L + 1 - f_l0[i]) * (d.ngrp - f_ist[i]));
+  }
+  SLE_TRY(upload(items, by_work(work), &set.ana_items));
+  // synthesis blocks: (order, latitude tile) with the tile's significant pieces
+  const int na = syn_na(d), ntile = (d.ngrp + na - 1) / na;
+  items.clear();
+  work.clear();
+  for (int m = 0; m < d.nm; ++m) {
+    for (int t = 0; t < ntile; ++t) {
+      const int glo = na * t, ghi = std::min(glo + na, d.ngrp) - 1;
+      uint32_t full = 0, half = 0;
+      long long c = 0;
+      for (int i = foff[m]; i < foff[m + 1]; ++i) {
+        if (f_ist[i] > ghi) continue;
+        const bool upper = na > 1 && f_ist[i] >= glo + na / 2;
+        (upper ? half : full) |= 1u << (i - foff[m]);
+        c += (long long)std::min(set.fseg, L + 1 - f_l0[i]) * (upper ? 1 : 2);
+      }
+      items.push_back(make_int4(m, t, (int)full, (int)half));
+      work.push_back(c);
+    }
+  }
+  return upload(items, by_work(work), &set.syn_items);
 }
 
 static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
@@ -888,7 +1003,6 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   SLE_TRY(dalloc(&p->segoff, d.nm + 1));
   SLE_TRY(dalloc(&p->seg_m, d.nseg));
   SLE_TRY(dalloc(&p->seg_l0, d.nseg));
-  SLE_TRY(dalloc(&p->ana_items, d.nseg));
   SLE_TRY(dalloc(&p->seeds, (size_t)d.nseg * d.nh));
   SLE_TRY(dalloc(&p->be, d.ncoef));
   SLE_TRY(dalloc(&p->cf, d.ncoef));
@@ -947,7 +1061,6 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   d.be = p->be;
   d.cf = p->cf;
   d.istart = p->istart;
-  d.ana_items = p->ana_items;
   d.tw = p->tw;
   d.X = p->X;
   d.EO = p->EO;
@@ -983,64 +1096,40 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   SLE_CUDA(cudaMemcpy(ist.data(), p->istart, d.nseg, cudaMemcpyDeviceToHost));
   cudaFree(segmax);
   cudaFree(fail);
-  // analysis order: most work first (segment length x active latitude groups)
-  std::vector<int> order(d.nseg);
-  std::iota(order.begin(), order.end(), 0);
-  std::vector<long long> work(d.nseg);
   long long done = 0, total = 0;
-  for (int s = 0; s < d.nseg; ++s) {
-    const int len = std::min(SEG, lmax + 1 - seg_l0[s]);
-    work[s] = (long long)len * (d.ngrp - ist[s]);
-    done += work[s];
+  for (int sg = 0; sg < d.nseg; ++sg) {
+    const int len = std::min(SEG, lmax + 1 - seg_l0[sg]);
+    done += (long long)len * (d.ngrp - ist[sg]);
     total += (long long)len * d.ngrp;
   }
   p->work_frac = total ? (double)done / (double)total : 1.0;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work[a] > work[b]; });
-  {
-    std::vector<int4> items(d.nseg);
-    for (int i = 0; i < d.nseg; ++i) items[i] = make_int4(order[i], seg_m[order[i]], seg_l0[order[i]], ist[order[i]]);
-    SLE_CUDA(cudaMemcpy(p->ana_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  }
-  {
-    // synthesis blocks: (order, latitude tile) with the tile's significant segments, most work first
-    const int na = syn_na(d), ntile = (d.ngrp + na - 1) / na;
-    std::vector<int4> items;
-    std::vector<long long> cost;
-    for (int m = 0; m < d.nm; ++m) {
-      for (int t = 0; t < ntile; ++t) {
-        const int glo = na * t, ghi = std::min(glo + na, d.ngrp) - 1;
-        uint32_t full = 0, half = 0;
-        long long c = 0;
-        for (int k = 0; segoff[m] + k < segoff[m + 1]; ++k) {
-          const int g = ist[segoff[m] + k];
-          if (g > ghi) continue;
-          const bool upper = na > 1 && g >= glo + na / 2;
-          (upper ? half : full) |= 1u << k;
-          c += (long long)std::min(SEG, lmax + 1 - seg_l0[segoff[m] + k]) * (upper ? 1 : 2);
-        }
-        items.push_back(make_int4(m, t, (int)full, (int)half));
-        cost.push_back(c);
-      }
-    }
-    std::vector<int> by(items.size());
-    std::iota(by.begin(), by.end(), 0);
-    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    std::vector<int4> sorted;
-    for (int i : by) sorted.push_back(items[i]);
-    SLE_TRY(dalloc(&p->syn_items, sorted.size()));
-    SLE_CUDA(cudaMemcpy(p->syn_items, sorted.data(), sorted.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    d.syn_items = p->syn_items;
-  }
+  SLE_TRY(leg_set_build(p, p->leg[0], 1, segoff, ist));
+  // shorter pieces (ana_set): a quarter or half of a segment while that
+  // leaves at most 12 warps per SM for one field
+  const int split = 4 * d.nseg <= 12 * p->n_sm ? 4 : 2 * d.nseg <= 12 * p->n_sm ? 2 : 1;
+  p->leg[1] = p->leg[0];
+  if (split > 1) SLE_TRY(leg_set_build(p, p->leg[1], split, segoff, ist));
 
 #define SLE_ATTR_FFT(NN)                                                                              \
   do {                                                                                                \
     SLE_CUDA(cudaFuncSetAttribute(k_fft_fold<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fft_smem(d)));    \
     SLE_CUDA(cudaFuncSetAttribute(k_ifft_unfold<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fft_smem(d))); \
-    SLE_CUDA(cudaFuncSetAttribute(k_fft_fold<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));               \
-    SLE_CUDA(cudaFuncSetAttribute(k_ifft_unfold<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));            \
+    SLE_CUDA(cudaFuncSetAttribute(k_fft_fold<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT));               \
+    SLE_CUDA(cudaFuncSetAttribute(k_ifft_unfold<NN>, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT));            \
   } while (0)
   SLE_FFT_SWITCH(d.n2, SLE_ATTR_FFT)
 #undef SLE_ATTR_FFT
+#define SLE_CARVE(...) \
+  SLE_CUDA(cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT))
+  SLE_CARVE(k_leg_ana<1>);
+  SLE_CARVE(k_leg_ana<2>);
+  SLE_CARVE(k_leg_syn<1, 1>);
+  SLE_CARVE(k_leg_syn<1, 2>);
+  SLE_CARVE(k_leg_syn<2, 1>);
+  SLE_CARVE(k_leg_syn<2, 2>);
+  SLE_CARVE(k_leg_syn<4, 1>);
+  SLE_CARVE(k_leg_syn<4, 2>);
+#undef SLE_CARVE
   SLE_CUDA(cudaDeviceSynchronize());
   return SLE_OK;
 }

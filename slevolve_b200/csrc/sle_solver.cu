@@ -1875,6 +1875,13 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, sle_batch** out) {
     const char* e = std::getenv("SLEVOLVE_B200_HOST_LOOP");
     s->use_graph = !(e && e[0] == '1');
   }
+  const void* kernels[] = {(const void*)k_step_begin, (const void*)k_advance, (const void*)k_ice_grid, (const void*)k_pre_spec,
+                           (const void*)k_rotation, (const void*)k_b18, (const void*)k_update, (const void*)k_sltot,
+                           (const void*)k_refresh1, (const void*)k_refresh2, (const void*)k_refresh2_x8, (const void*)k_dice,
+                           (const void*)k_loop_cond, (const void*)k_reopen, (const void*)k_rr, (const void*)k_commit,
+                           (const void*)k_post_grid, (const void*)k_diag00};
+  for (const void* k : kernels)
+    TRYC(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, SMEM_CARVEOUT));
   // K00 = synth(e00)[0,0] (solver_opt.py:320-325): the same for every slot of the grid
   s->K00 = 0.0;
   if (cfg->opt_dsl) {
