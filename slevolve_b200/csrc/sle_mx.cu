@@ -30,7 +30,7 @@
 // one half each (a launch-shape choice), a half being one parity of one 32-wide K chunk):
 //   warp 13     loader: per half, one bulk copy of the FP32 A tile (16 KB) and the B data
 //               (analysis: one 4-D TMA tensor load of the folded FFT; synthesis: one bulk copy)
-//               into stage q % stages
+//               into stage q % stages (analysis: landing slot q % (stages + 2))
 //   warps 4-11  splitters, group g takes the halves q = g mod 2: the TF32 lo tiles of A and B
 //               (the FP32 tiles serve as hi; the analysis B box is first moved to the hi tile)
 //   warp 12     allocates TMEM and issues the MMAs from one thread: a unit's halves of parity 0
@@ -62,11 +62,24 @@ constexpr int TILE_F = 128 * KC;              // words of one A tile (128 rows x
 constexpr int TILE_A = TILE_F * 4;            // 16 KB
 constexpr int SLOT_WORDS = 2 * TILE_F;        // Legendre table slot: FP32 A tiles of both parities
 constexpr int TILE_B = MX_NMAX * 128;         // MX_NMAX rows x 128 bytes = 8 KB
-constexpr int STAGE_BYTES = 2 * TILE_A + 2 * TILE_B;   // one parity of a chunk: A hi / lo, B hi / lo
+constexpr int STAGE_BYTES = 2 * TILE_A + 2 * TILE_B;   // synthesis: one parity of a chunk, A hi / lo, B hi / lo
 constexpr int NSTAGE_MAX = 4;                 // pipeline stages: 2 or 4 (a launch-time choice)
+// analysis: landing slots (the A tile, which serves as A hi, and the B box) and work slots (A lo, B hi,
+// B lo), an even number of each: stages + 2 and 2 in the deep form, 4 and 4 in the wide one
+constexpr int RAW_BYTES = TILE_A + TILE_B;
+constexpr int WORK_BYTES = TILE_A + 2 * TILE_B;
+constexpr int NRAW_MAX = NSTAGE_MAX + 2;
+constexpr int NWORK_MAX = 2;                   // work slots with a barrier of their own (deep form)
+__host__ __device__ constexpr int raw_slots(bool syn, int nst, bool deep) { return syn ? nst : deep ? nst + 2 : 4; }
+__host__ __device__ constexpr int work_slots(bool deep) { return deep ? 2 : 4; }
+__host__ __device__ constexpr int pipe_bytes(bool syn, int nst, bool deep) {
+  return syn ? nst * STAGE_BYTES : raw_slots(syn, nst, deep) * RAW_BYTES + work_slots(deep) * WORK_BYTES;
+}
 constexpr int MISC_BYTES = 1024;              // barriers + bookkeeping
 constexpr int EVEN_BYTES = 128 * MX_NMAX * 4;   // synthesis: the even-degree sums of a unit (FP32, 128 rows)
-constexpr int mx_smem(int nst, bool syn = false) { return 1024 + nst * STAGE_BYTES + MISC_BYTES + (syn ? EVEN_BYTES : 0); }
+constexpr int mx_smem(int nst, bool syn, bool deep) {
+  return 1024 + pipe_bytes(syn, nst, deep) + MISC_BYTES + (syn ? EVEN_BYTES : 0);
+}
 constexpr int W_SPL = 4;                      // warps 4..11: splitters (two groups of four)
 constexpr int W_MMA = 12;                     // TMEM owner, MMA issue
 constexpr int W_LOAD = 13;                    // bulk / TMA loads
@@ -87,8 +100,9 @@ constexpr double SYN_UNIT_COST = 24.0;
 constexpr int NCOLS = MX_NMAX;                // accumulator columns of every launch (2 per field slot)
 static_assert(512 + 16 * MAX_CTA_UNITS <= MISC_BYTES, "misc shared memory too small");
 
-static_assert(NSTAGE_MAX % 2 == 0, "a stage must always hold halves of one parity");
-static_assert(mx_smem(NSTAGE_MAX, true) <= 232448, "mixed transform shared memory exceeds the sm_100a limit");
+static_assert(NSTAGE_MAX % 2 == 0 && NRAW_MAX % 2 == 0, "a stage must always belong to one splitter group");
+static_assert(mx_smem(NSTAGE_MAX, true, true) <= 232448 && mx_smem(NSTAGE_MAX, false, true) <= 232448 &&
+                  mx_smem(NSTAGE_MAX, false, false) <= 232448, "mixed transform shared memory exceeds the sm_100a limit");
 static_assert(TILE_B == MX_NMAX * 128, "full-width MMAs read B hi and B lo as one tile of 2 MX_NMAX rows");
 static_assert(2 * NPAIR * 2 * MX_NMAX <= (int)TMEM_COLS && NPAIR * 2 * MX_NMAX == (int)PAR_COLS,
               "accumulators exceed TMEM");
@@ -147,22 +161,6 @@ __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-__device__ __forceinline__ void named_bar(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// AND of `v` over the `n` threads that reach named barrier `id` (all of them must).
-__device__ __forceinline__ bool bar_and(int id, int n, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, %2, %3, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
-}
-
 __device__ __forceinline__ void tc_alloc(uint32_t holder, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(holder), "r"(ncols)
                : "memory");
@@ -219,10 +217,11 @@ __host__ __device__ __forceinline__ int sw_off(int row, int k) {
 // ------------------------------------------------------------- precision splits
 // The lo part for a hi part that is x itself read as TF32: a kind::tf32 MMA ignores the 13 low
 // mantissa bits of an FP32 operand, so x serves as hi = trunc(x) unchanged and only
-// lo = TF32(x - trunc(x)) is written (|x - trunc(x) - lo| <= 2^-21 |x|).
+// lo = TF32(x - trunc(x)) is written (|x - trunc(x) - lo| <= 2^-21 |x|), rounded to nearest by adding
+// half of the 13 bits' range; the bits below are left as they are, the MMA ignores them here too.
 __device__ __forceinline__ uint32_t lo_of_trunc(float x) {
   const float r = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-  return (__float_as_uint(r) + 0x1000u) & 0xFFFFE000u;
+  return __float_as_uint(r) + 0x1000u;
 }
 
 // ------------------------------------------------------------------ bounded waits
@@ -293,36 +292,50 @@ __device__ __forceinline__ bool field_off(const MxFieldArgs& a, int f) {
   return false;
 }
 
-// Shared memory of a stage (one parity of one chunk): A tiles [hi][lo] (the parity's FP32
-// Legendre tile lands in hi and is split in place), then B tiles [hi][lo] (the raw B data lands
-// in lo).
+// Shared memory of half q.  Synthesis: stage q % NST holds the A tiles [hi][lo] (the parity's FP32
+// Legendre tile lands in hi and serves as hi) and the B tiles [hi][lo] (the raw B data lands in hi).
+// Analysis: landing slot q % NR holds the A tile and the folded FFT's box, work slot q & 1 the tiles
+// that the splitters write.  The landing slots are half as large as a stage, so that in the deep form
+// six halves' loads are in flight: with four, the loader waited two thirds of the time for a slot and
+// the splitters almost half of it for a load (five to seven units per CTA).
+template <bool SYN, int NST, bool DEEP>
 struct Smem {
+  static constexpr int NR = raw_slots(SYN, NST, DEEP);
+  static constexpr int NW = SYN ? NST : work_slots(DEEP);
   uint8_t* base;        // generic pointer, 1024-aligned
   uint32_t sbase;       // shared-window address of base
-  int nst;              // stages of this launch
-  __device__ uint32_t a_tile(int stage, int lo) const { return sbase + stage * STAGE_BYTES + lo * TILE_A; }
-  __device__ uint8_t* a_ptr(int stage, int lo) const { return base + stage * STAGE_BYTES + lo * TILE_A; }
-  __device__ uint32_t b_tile(int stage, int lo) const {
-    return sbase + stage * STAGE_BYTES + 2 * TILE_A + lo * TILE_B;
-  }
-  __device__ uint8_t* b_ptr(int stage, int lo) const { return base + stage * STAGE_BYTES + 2 * TILE_A + lo * TILE_B; }
-  __device__ uint8_t* misc() const { return base + nst * STAGE_BYTES; }
-  __device__ float* even() const { return reinterpret_cast<float*>(base + nst * STAGE_BYTES + MISC_BYTES); }
+  __device__ static int raw_off(int q) { return SYN ? (q % NST) * STAGE_BYTES : (q % NR) * RAW_BYTES; }
+  __device__ static int work_off(int q) { return NR * RAW_BYTES + (q % NW) * WORK_BYTES; }
+  __device__ static int a_hi(int q) { return raw_off(q); }
+  __device__ static int a_lo(int q) { return SYN ? raw_off(q) + TILE_A : work_off(q); }
+  __device__ static int b_box(int q) { return raw_off(q) + TILE_A; }   // analysis
+  __device__ static int b_hi(int q) { return SYN ? raw_off(q) + 2 * TILE_A : work_off(q) + TILE_A; }
+  __device__ static int b_lo(int q) { return b_hi(q) + TILE_B; }
+  // barrier of the splitters' hand-over of half q, and its phase parity
+  __device__ static int full(int q) { return q % NW; }
+  __device__ static uint32_t full_phase(int q) { return (uint32_t)((q / NW) & 1); }
+  __device__ uint32_t at(int off) const { return sbase + off; }
+  template <typename T>
+  __device__ T* ptr(int off) const { return reinterpret_cast<T*>(base + off); }
+  __device__ uint8_t* misc() const { return base + pipe_bytes(SYN, NST, DEEP); }
+  __device__ float* even() const { return reinterpret_cast<float*>(base + pipe_bytes(SYN, NST, DEEP) + MISC_BYTES); }
 };
 
-__device__ __forceinline__ Smem smem_layout(uint8_t* raw, int nst) {
+template <bool SYN, int NST, bool DEEP>
+__device__ __forceinline__ Smem<SYN, NST, DEEP> smem_layout(uint8_t* raw) {
   const uint32_t s = smem_u32(raw);
   const uint32_t al = (s + 1023u) & ~1023u;
-  return Smem{raw + (al - s), al, nst};
+  return Smem<SYN, NST, DEEP>{raw + (al - s), al};
 }
 
-// Barriers: full[nst] (splitters -> MMA), empty[nst] (MMA commit -> loader), raw[nst] (copies
-// landed -> splitters), accum[2] (a unit's MMAs of one parity done -> epilogue), tfree[2]
-// (epilogue done reading that parity's accumulators -> MMA), drain (MMAs issued before an
-// abort); each stage group has room for the largest stage count.
-enum { BAR_FULL = 0, BAR_EMPTY = NSTAGE_MAX, BAR_RAW = 2 * NSTAGE_MAX, BAR_ACCUM = 3 * NSTAGE_MAX,
-       BAR_TFREE = 3 * NSTAGE_MAX + 2, BAR_DRAIN = 3 * NSTAGE_MAX + 4, NBAR = 3 * NSTAGE_MAX + 5 };
-static_assert(NBAR * 8 <= 192, "barrier area too small");
+// Barriers: full[] (splitters -> MMA; per stage, in the analysis per work slot), empty[] (MMA commit ->
+// loader), raw[] (copies landed -> splitters), wfree[] (analysis: MMA commit -> splitters, the work slot
+// is free), accum[2] (a unit's MMAs of one parity done -> epilogue), tfree[2] (epilogue done reading
+// that parity's accumulators -> MMA), drain (MMAs issued before an abort); each group has room for the
+// largest stage count.
+enum { BAR_FULL = 0, BAR_EMPTY = NSTAGE_MAX, BAR_RAW = BAR_EMPTY + NRAW_MAX, BAR_WFREE = BAR_RAW + NRAW_MAX,
+       BAR_ACCUM = BAR_WFREE + NWORK_MAX, BAR_TFREE = BAR_ACCUM + 2, BAR_DRAIN = BAR_TFREE + 2, NBAR = BAR_DRAIN + 1 };
+static_assert(NBAR * 8 <= 224, "barrier area too small");
 static_assert(MX_MAXF == 32, "the launch's active fields are one 32-bit mask");
 struct Misc {
   uint64_t* bar;
@@ -331,11 +344,10 @@ struct Misc {
   int4* units;          // [MAX_CTA_UNITS]: this CTA's work units, staged by the prologue
   __device__ uint32_t b(int i) const { return smem_u32(bar + i); }
 };
-__device__ __forceinline__ Misc misc_layout(const Smem& S) {
-  uint8_t* p = S.misc();
+__device__ __forceinline__ Misc misc_layout(uint8_t* p) {
   Misc m;
-  m.bar = reinterpret_cast<uint64_t*>(p);                      // 17 barriers
-  m.tmem_holder = reinterpret_cast<uint32_t*>(p + 192);
+  m.bar = reinterpret_cast<uint64_t*>(p);                      // NBAR barriers
+  m.tmem_holder = reinterpret_cast<uint32_t*>(p + 224);
   m.any = reinterpret_cast<int*>(p + 256);
   m.units = reinterpret_cast<int4*>(p + 512);
   return m;
@@ -350,13 +362,14 @@ __device__ __forceinline__ Misc misc_layout(const Smem& S) {
 // parity-0 halves first, then its parity-1 halves: while the epilogue drains one parity's half of
 // TMEM, the MMAs of the other parity run.
 
-// MMAs of one parity `par` of chunk k of a unit (stage st): four K steps of 8, each one
+// MMAs of one parity `par` of chunk k of a unit (half q): four K steps of 8, each one
 // M128 x N128 MMA (Ahi [Bhi | Blo] into [main | correction]) and one M128 x N64 (Alo Bhi into the
 // correction).  The K sub-block kk starts 32 kk bytes into the tile rows: +2 kk in the
 // descriptor's start-address field.
-__device__ __forceinline__ void mma_half(const Smem& S, uint32_t tmem, int st, int par, int k) {
-  const uint64_t ah = sdesc_sw128(S.a_tile(st, 0)), al = sdesc_sw128(S.a_tile(st, 1));
-  const uint64_t bh = sdesc_sw128(S.b_tile(st, 0));
+template <typename SM>
+__device__ __forceinline__ void mma_half(const SM& S, uint32_t tmem, int q, int par, int k) {
+  const uint64_t ah = sdesc_sw128(S.at(S.a_hi(q))), al = sdesc_sw128(S.at(S.a_lo(q)));
+  const uint64_t bh = sdesc_sw128(S.at(S.b_hi(q)));
   const uint32_t idesc = idesc_tf32(128, NCOLS), idesc2 = idesc_tf32(128, 2 * NCOLS);
   // B hi rows [0, N) and B lo rows [0, N) are 2N consecutive rows (TILE_B = N rows)
   const uint32_t dm = tmem + PAR_COLS * (uint32_t)par + (uint32_t)(2 * NCOLS * (k % NPAIR));
@@ -395,16 +408,17 @@ __device__ __forceinline__ void acc_read(uint32_t base, int nch, int cb, double 
 }
 
 // Common prologue: barriers, gates, TMEM.  Returns the TMEM base (all threads).
-__device__ uint32_t prologue(const Smem& S, const Misc& M, const MxFieldArgs& a, const int4* units, int2 rg,
+__device__ uint32_t prologue(int nfull, int nraw, const Misc& M, const MxFieldArgs& a, const int4* units, int2 rg,
                              int tfree_warps) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x < MAX_CTA_UNITS && (int)threadIdx.x < rg.y) M.units[threadIdx.x] = units[rg.x + threadIdx.x];
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S.nst; ++i) {
-      mbar_init(M.b(BAR_FULL + i), 4);    // the 4 splitter warps of the stage
+    for (int i = 0; i < nfull; ++i) mbar_init(M.b(BAR_FULL + i), 4);   // the 4 warps of a splitter group
+    for (int i = 0; i < nraw; ++i) {
       mbar_init(M.b(BAR_EMPTY + i), 1);   // one tcgen05.commit
       mbar_init(M.b(BAR_RAW + i), 1);     // loader's expect_tx
     }
+    for (int i = 0; i < NWORK_MAX; ++i) mbar_init(M.b(BAR_WFREE + i), 1);   // one tcgen05.commit
     for (int i = 0; i < 2; ++i) {
       mbar_init(M.b(BAR_ACCUM + i), 1);   // one tcgen05.commit (or arrive for an empty unit)
       mbar_init(M.b(BAR_TFREE + i), tfree_warps);   // the epilogue warps that read the parity
@@ -522,10 +536,8 @@ __global__ void __launch_bounds__(128) k_tab_syn(ShtDev P, uint32_t* tab) {
 // A split: the FP32 Legendre values landed in the hi tile of the stage and serve as hi as they
 // are (the MMA reads them as TF32, trunc(x)); the lo tile gets TF32(x - trunc(x)).  Elementwise,
 // so the tile order does not matter.
-__device__ __forceinline__ void split_a(const Smem& S, int st, int tid) {
+__device__ __forceinline__ void split_a(const uint4* hp, uint4* lp, int tid) {
   constexpr int NV = TILE_F / 4 / 128;   // 16-byte vectors per thread
-  const uint4* hp = reinterpret_cast<const uint4*>(S.a_ptr(st, 0));
-  uint4* lp = reinterpret_cast<uint4*>(S.a_ptr(st, 1));
   uint4 v[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) v[q] = hp[tid + 128 * q];
@@ -536,40 +548,32 @@ __device__ __forceinline__ void split_a(const Smem& S, int st, int tid) {
 }
 
 // Analysis B data of one parity: the TMA box of the folded FFT is [field][32 latitudes][re, im]
-// (8 bytes per entry) in the stage's B lo tile; the 4 splitter warps read it, synchronise, and
-// write rows 2f (re) / 2f+1 (im) of the B hi tile (the FP32 values, read as TF32 by the MMA)
-// and of the B lo tile (TF32 of x - trunc(x)).
-__device__ __forceinline__ void split_b_ana(const Smem& S, int st, int nf, int tid, int bar_id) {
-  const float2* box = reinterpret_cast<const float2*>(S.b_ptr(st, 1));
-  float2 v[8];
+// (8 bytes per entry) in the landing slot; the 4 splitter warps write rows 2f (re) / 2f+1 (im) of
+// the B hi tile (the FP32 values, read as TF32 by the MMA) and of the B lo tile (TF32 of
+// x - trunc(x)), four latitudes (16 bytes of a row) at a time.
+__device__ __forceinline__ void split_b_ana(const uint4* box, uint4* hp, uint4* lp, int nf, int tid) {
 #pragma unroll
-  for (int u = 0; u < 8; ++u) {
+  for (int u = 0; u < MX_MAXF / 16; ++u) {
     const int e = tid + 128 * u;
-    v[u] = ((e >> 5) < nf) ? box[e] : make_float2(0.f, 0.f);
-  }
-  named_bar(bar_id, 128);
-  uint32_t* hp = reinterpret_cast<uint32_t*>(S.b_ptr(st, 0));
-  uint32_t* lp = reinterpret_cast<uint32_t*>(S.b_ptr(st, 1));
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int e = tid + 128 * u;
-    const int f = e >> 5, k = e & 31;
+    const int f = e >> 3, c = e & 7;   // field, 16-byte chunk of the row
     if (f >= nf) continue;
-    const int o0 = sw_off(2 * f, k), o1 = sw_off(2 * f + 1, k);
-    hp[o0] = __float_as_uint(v[u].x);
-    lp[o0] = lo_of_trunc(v[u].x);
-    hp[o1] = __float_as_uint(v[u].y);
-    lp[o1] = lo_of_trunc(v[u].y);
+    const uint4 x = box[2 * e], y = box[2 * e + 1];
+    const int r0 = 2 * f, r1 = r0 + 1;
+    const int o0 = r0 * (KC / 4) + (c ^ (r0 & 7)), o1 = r1 * (KC / 4) + (c ^ (r1 & 7));
+    hp[o0] = make_uint4(x.x, x.z, y.x, y.z);
+    hp[o1] = make_uint4(x.y, x.w, y.y, y.w);
+    lp[o0] = make_uint4(lo_of_trunc(__uint_as_float(x.x)), lo_of_trunc(__uint_as_float(x.z)),
+                        lo_of_trunc(__uint_as_float(y.x)), lo_of_trunc(__uint_as_float(y.z)));
+    lp[o1] = make_uint4(lo_of_trunc(__uint_as_float(x.y)), lo_of_trunc(__uint_as_float(x.w)),
+                        lo_of_trunc(__uint_as_float(y.y)), lo_of_trunc(__uint_as_float(y.w)));
   }
 }
 
 // Synthesis B data of one parity: the raw block lands in the hi tile, already in the tile order,
 // and serves as hi as it is; the lo tile gets TF32(x - trunc(x)).  16-byte vectors; the rows beyond
 // the launch's fields hold whatever the stage held before (their columns are not read).
-__device__ __forceinline__ void split_b_syn(const Smem& S, int st, int nrow, int tid) {
+__device__ __forceinline__ void split_b_syn(const uint4* hp, uint4* lp, int nrow, int tid) {
   constexpr int NV = TILE_B / 16 / 128;   // 16-byte vectors per thread of a full tile
-  const uint4* hp = reinterpret_cast<const uint4*>(S.b_ptr(st, 0));
-  uint4* lp = reinterpret_cast<uint4*>(S.b_ptr(st, 1));
   uint4 v[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q)
@@ -627,20 +631,23 @@ __device__ __forceinline__ void degree0(const ShtDev& P, const Misc& M, const Mx
 // parity); warp 12 issues the MMAs of a unit's parity p once the epilogue has read parity p of
 // the unit before out of TMEM; warps 0-3 and 14-17 drain the unit (analysis: one parity per
 // group; synthesis: one half of the fields per group, both parities).
-template <bool SYN, int NST>
+template <bool SYN, int NST, bool DEEP>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_leg_tc(ShtDev P, MxFieldArgs a, int* status, const __grid_constant__ CUtensorMap tmx, int zbox) {
   static_assert(NST % 2 == 0 && NST <= NSTAGE_MAX, "stage count");
   extern __shared__ uint8_t smraw[];
-  const Smem S = smem_layout(smraw, NST);
-  const Misc M = misc_layout(S);
+  using SM = Smem<SYN, NST, DEEP>;
+  const SM S = smem_layout<SYN, NST, DEEP>(smraw);
+  constexpr int NR = SM::NR, NW = SM::NW;
+  static_assert(NR % 2 == 0 && NW % 2 == 0, "a slot must always belong to one splitter group");
+  const Misc M = misc_layout(S.misc());
   const Abort ab{P.mx_abort, P.mx_abort_host, status};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int L = P.lmax;
   const uint32_t* tab = SYN ? P.mx_tab_syn : P.mx_tab_ana;
   // this CTA's work units: rg.y units from rg.x on (the plan balances the CTAs' totals)
   const int2 rg = (SYN ? P.mx_syn_cta : P.mx_ana_cta)[blockIdx.x];
-  const uint32_t tmem = prologue(S, M, a, SYN ? P.mx_syn_units : P.mx_ana_units, rg, SYN ? 8 : 4);
+  const uint32_t tmem = prologue(NW, NR, M, a, SYN ? P.mx_syn_units : P.mx_ana_units, rg, SYN ? 8 : 4);
   if (*M.any && *reinterpret_cast<volatile int*>(P.mx_abort) == 0) {
     const int nrow = 2 * a.nf;
     const uint32_t act = (uint32_t)*M.any;   // bit f: field f is active
@@ -655,26 +662,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           int nch;
           unit_info<SYN>(P, M, u, i, unit, nch);
           for (int h = 0; h < 2 * nch; ++h, ++q) {
-            const int par = h >= nch ? 1 : 0, k = h - par * nch, st = q % NST;
-            if (!mbar_spin(M.b(BAR_EMPTY + st), (uint32_t)(((q / NST) & 1) ^ 1), ab)) {
+            const int par = h >= nch ? 1 : 0, k = h - par * nch, st = q % NR;
+            if (!mbar_spin(M.b(BAR_EMPTY + st), (uint32_t)(((q / NR) & 1) ^ 1), ab)) {
               ok = false;
               break;
             }
             const uint32_t raw = M.b(BAR_RAW + st);
             mbar_arrive_expect_tx(raw, (uint32_t)TILE_A + bbytes);
-            bulk_g2s(S.a_tile(st, 0), tab + ((long long)unit.w + k) * SLOT_WORDS + par * TILE_F, (uint32_t)TILE_A,
+            bulk_g2s(S.at(S.a_hi(q)), tab + ((long long)unit.w + k) * SLOT_WORDS + par * TILE_F, (uint32_t)TILE_A,
                      raw);
             if (SYN) {
               const int seg = P.mx_syn_seg[unit.w + k];
-              bulk_g2s(S.b_tile(st, 0), P.mx_bsyn + ((size_t)seg * 2 + par) * BBLOCK, (uint32_t)nrow * 128u, raw);
+              bulk_g2s(S.at(S.b_hi(q)), P.mx_bsyn + ((size_t)seg * 2 + par) * BBLOCK, (uint32_t)nrow * 128u, raw);
             } else {
-              tma_load_4d(S.b_tile(st, 1), &tmx, 2 * KC * (unit.z + k), par, unit.x, 0, raw);
+              tma_load_4d(S.at(S.b_box(q)), &tmx, 2 * KC * (unit.z + k), par, unit.x, 0, raw);
             }
           }
         }
         // copies in flight land before the CTA exits: the last phase issued on each stage
-        for (int st = 0; st < NST; ++st) {
-          const int n_st = (q + NST - 1 - st) / NST;   // loads issued on stage st
+        for (int st = 0; st < NR; ++st) {
+          const int n_st = (q + NR - 1 - st) / NR;   // loads issued on slot st
           if (n_st > 0) mbar_wait_drain(M.b(BAR_RAW + st), (uint32_t)((n_st - 1) & 1));
         }
       }
@@ -694,15 +701,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             }
             tc_fence_after();
             for (int k = 0; k < nch; ++k, ++q) {
-              const int st = q % NST;
-              if (!mbar_spin(M.b(BAR_FULL + st), (uint32_t)((q / NST) & 1), ab)) {
+              if (!mbar_spin(M.b(BAR_FULL + S.full(q)), S.full_phase(q), ab)) {
                 ok = false;
                 break;
               }
               tc_fence_after();
-              mma_half(S, tmem, st, par, k);
+              mma_half(S, tmem, q, par, k);
               issued = true;
-              tc_commit(M.b(BAR_EMPTY + st));
+              tc_commit(M.b(BAR_EMPTY + q % NR));
+              if (NW != NR) tc_commit(M.b(BAR_WFREE + q % NW));
             }
             if (!ok) break;
             if (nch > 0) tc_commit(M.b(BAR_ACCUM + par));
@@ -727,20 +734,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         unit_info<SYN>(P, M, u, i, unit, nch);
         for (int h = 0; h < 2 * nch; ++h, ++q) {
           if ((q & 1) != g) continue;
-          const int st = q % NST;
-          // every wait is bounded, so all four warps of the group reach the vote; they go on
-          // (and meet at the named barrier of the B split) only together
-          const bool w = mbar_wait(M.b(BAR_RAW + st), (uint32_t)((q / NST) & 1), ab);
-          if (!bar_and(1 + g, 128, w)) {
+          // each warp of the group goes on by itself: it writes its own part of the tiles and arrives
+          // for it (a warp whose wait failed leaves; the MMA issuer's wait then runs out)
+          bool w = mbar_wait(M.b(BAR_RAW + q % NR), (uint32_t)((q / NR) & 1), ab);
+          // (with as many work as landing slots the two are freed together: the loader waited)
+          if (NW != NR) w = mbar_wait(M.b(BAR_WFREE + q % NW), S.full_phase(q) ^ 1u, ab) && w;
+          if (!__all_sync(0xffffffffu, w)) {
             ok = false;
             break;
           }
-          split_a(S, st, tid);
-          if (SYN) split_b_syn(S, st, nrow, tid);
-          else split_b_ana(S, st, a.nf, tid, 1 + g);
+          split_a(S.template ptr<const uint4>(S.a_hi(q)), S.template ptr<uint4>(S.a_lo(q)), tid);
+          if (SYN)
+            split_b_syn(S.template ptr<const uint4>(S.b_hi(q)), S.template ptr<uint4>(S.b_lo(q)), nrow, tid);
+          else
+            split_b_ana(S.template ptr<const uint4>(S.b_box(q)), S.template ptr<uint4>(S.b_hi(q)),
+                        S.template ptr<uint4>(S.b_lo(q)), a.nf, tid);
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0) mbar_arrive(M.b(BAR_FULL + st));
+          if (lane == 0) mbar_arrive(M.b(BAR_FULL + S.full(q)));
         }
       }
     } else if (SYN) {
@@ -1288,10 +1299,14 @@ int sht_mx_prepare(sle_sht* p) {
       return SLE_ERR_CUDA;
     }
   }
-  SLE_CUDA(cudaFuncSetAttribute(k_leg_tc<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx_smem(2)));
-  SLE_CUDA(cudaFuncSetAttribute(k_leg_tc<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx_smem(2, true)));
-  SLE_CUDA(cudaFuncSetAttribute(k_leg_tc<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx_smem(4)));
-  SLE_CUDA(cudaFuncSetAttribute(k_leg_tc<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx_smem(4, true)));
+#define SLE_ATTR_TC(SYN, NST, DEEP) \
+  SLE_CUDA(cudaFuncSetAttribute(k_leg_tc<SYN, NST, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx_smem(NST, SYN, DEEP)))
+  SLE_ATTR_TC(false, 2, true);
+  SLE_ATTR_TC(false, 4, true);
+  SLE_ATTR_TC(false, 4, false);
+  SLE_ATTR_TC(true, 2, true);
+  SLE_ATTR_TC(true, 4, true);
+#undef SLE_ATTR_TC
 #define SLE_ATTR_MX(NN)                                                                                        \
   do {                                                                                                         \
     SLE_CUDA(cudaFuncSetAttribute(k_fold_mx<NN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx_fold_smem(d, 4)));    \
@@ -1319,12 +1334,14 @@ static int mx_check_args(const MxFieldArgs& a, const char* what) {
   return SLE_OK;
 }
 
-// Whether a tensor-core launch of so many work units may be scheduled while the kernel before it is
-// finishing (programmatic launch; its prologue then overlaps that kernel's tail).  With at most two
-// units per CTA (up to L = 255) the prologue is a tenth of the launch: the 12-member batch step at L =
-// 127 takes 1162 us instead of 1201.  At L = 511 (five to seven units) the 32-member step was 1.2 %
-// slower with it (8117 against 8022 us).
-static bool tc_early(const sle_sht* p, int units) { return units <= 2 * p->n_sm; }
+// Whether a tensor-core launch has at most two work units per CTA (up to L = 255).  Its prologue is then a
+// tenth of the launch, and it is launched programmatically, so that the prologue overlaps the tail of the
+// kernel before: the 12-member batch step at L = 127 took 1162 us instead of 1201, but at L = 511 (five to
+// seven units) the 32-member step was 1.2 % slower with it (8117 against 8022 us).  And with few
+// halves per CTA the depth of the loads does not matter: the analysis takes the wide form there (12
+// fields at L = 127: 13.1 us wide, 14.4 deep), the deep one at L = 511 (32 fields: 78.7 us with four of
+// both, 75.4 deep; 5 fields 61.7 and 55.8).
+static bool tc_small(const sle_sht* p, int units) { return units <= 2 * p->n_sm; }
 
 int sht_mx_analysis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t st, int prof_cls) {
   SLE_TRY(sht_mx_prepare(p));
@@ -1346,12 +1363,14 @@ int sht_mx_analysis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t 
   const int zi = (a.nf <= ZBOX[0]) ? 0 : (a.nf <= ZBOX[1]) ? 1 : 2;
   const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(p->mx_tmap[zi]);
   ProfToken t1 = prof_begin(prof_cls, a.nf, st);
-  if (p->tune_stages == 2)
-    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_ana_units), k_leg_tc<false, 2>, dim3(p->n_ana_cta), dim3(TC_THREADS),
-                           mx_smem(2), st, d, a, status, *map, ZBOX[zi]));
-  else
-    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_ana_units), k_leg_tc<false, 4>, dim3(p->n_ana_cta), dim3(TC_THREADS),
-                           mx_smem(4), st, d, a, status, *map, ZBOX[zi]));
+  const bool small = tc_small(p, p->n_ana_units);
+#define SLE_LAUNCH_TC(NST, DEEP)                                                                           \
+  SLE_CUDA(launch_pdl_if(small, k_leg_tc<false, NST, DEEP>, dim3(p->n_ana_cta), dim3(TC_THREADS),          \
+                         mx_smem(NST, false, DEEP), st, d, a, status, *map, ZBOX[zi]))
+  if (p->tune_stages == 2) SLE_LAUNCH_TC(2, true);
+  else if (small) SLE_LAUNCH_TC(4, false);
+  else SLE_LAUNCH_TC(4, true);
+#undef SLE_LAUNCH_TC
   prof_end(t1, st);
   note_launch(2);
   SLE_CUDA(cudaGetLastError());
@@ -1365,12 +1384,12 @@ int sht_mx_synthesis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t
   const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(p->mx_tmap[0]);
   ProfToken t0 = prof_begin(PROF_LEG_SYN, a.nf, st);
   if (!b_ready) SLE_CUDA(launch_pdl(k_bsyn_mx, dim3(d.nseg, (a.nf + 3) / 4), dim3(256), 0, st, d, a));
-  if (p->tune_stages == 2)
-    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_syn_units), k_leg_tc<true, 2>, dim3(p->n_syn_cta), dim3(TC_THREADS),
-                           mx_smem(2, true), st, d, a, status, *map, 0));
-  else
-    SLE_CUDA(launch_pdl_if(tc_early(p, p->n_syn_units), k_leg_tc<true, 4>, dim3(p->n_syn_cta), dim3(TC_THREADS),
-                           mx_smem(4, true), st, d, a, status, *map, 0));
+#define SLE_LAUNCH_TC(NST)                                                                                  \
+  SLE_CUDA(launch_pdl_if(tc_small(p, p->n_syn_units), k_leg_tc<true, NST, true>, dim3(p->n_syn_cta),        \
+                         dim3(TC_THREADS), mx_smem(NST, true, true), st, d, a, status, *map, 0))
+  if (p->tune_stages == 2) SLE_LAUNCH_TC(2);
+  else SLE_LAUNCH_TC(4);
+#undef SLE_LAUNCH_TC
   prof_end(t0, st);
   ProfToken t1 = prof_begin(PROF_IFFT, a.nf, st);
 #define SLE_LAUNCH_MXU(NN) \
