@@ -283,6 +283,7 @@ struct sle_sht {
   int n_ana_units, n_syn_units;
   int n_ana_cta, n_syn_cta;       // CTAs of an analysis / synthesis launch
   int n_sm;                      // SMs of the device
+  bool early;                    // launch the transforms' kernels programmatically
   // blocks of the unfold resident on the device at once (occupancy x SMs): each block prefetches
   // into L2 the input of the block that many places further on in launch order
   int unfold_ahead;

@@ -1380,7 +1380,7 @@ int sht_mx_analysis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t 
   ProfToken t1 = prof_begin(prof_cls, a.nf, st);
   const bool small = tc_small(p, p->n_ana_units);
 #define SLE_LAUNCH_TC(NST, DEEP)                                                                           \
-  SLE_CUDA(launch_pdl_if(small, k_leg_tc<false, NST, DEEP>, dim3(p->n_ana_cta), dim3(TC_THREADS),          \
+  SLE_CUDA(launch_pdl_if(p->early && small, k_leg_tc<false, NST, DEEP>, dim3(p->n_ana_cta), dim3(TC_THREADS),          \
                          mx_smem(NST, false, DEEP), st, d, a, status, *map, ZBOX[zi]))
   if (p->tune_stages == 2) SLE_LAUNCH_TC(2, true);
   else if (small) SLE_LAUNCH_TC(4, false);
@@ -1398,9 +1398,9 @@ int sht_mx_synthesis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t
   const ShtDev& d = p->d;
   const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(p->mx_tmap[0]);
   ProfToken t0 = prof_begin(PROF_LEG_SYN, a.nf, st);
-  if (!b_ready) SLE_CUDA(launch_pdl(k_bsyn_mx, dim3(d.nseg, (a.nf + 7) / 8), dim3(256), 0, st, d, a));
+  if (!b_ready) SLE_CUDA(launch_pdl_if(p->early, k_bsyn_mx, dim3(d.nseg, (a.nf + 7) / 8), dim3(256), 0, st, d, a));
 #define SLE_LAUNCH_TC(NST)                                                                                  \
-  SLE_CUDA(launch_pdl_if(tc_small(p, p->n_syn_units), k_leg_tc<true, NST, true>, dim3(p->n_syn_cta),        \
+  SLE_CUDA(launch_pdl_if(p->early && tc_small(p, p->n_syn_units), k_leg_tc<true, NST, true>, dim3(p->n_syn_cta),        \
                          dim3(TC_THREADS), mx_smem(NST, true, true), st, d, a, status, *map, 0))
   if (p->tune_stages == 2) SLE_LAUNCH_TC(2);
   else SLE_LAUNCH_TC(4);

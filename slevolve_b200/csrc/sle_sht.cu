@@ -714,9 +714,9 @@ static int fp64_leg_ana(const sle_sht* plan, ShtDev d, const SpecPtrs& o, int nf
   d.leg = ana_set(plan, nf);
   const unsigned gx = (unsigned)((d.leg.nfseg + ANA_WARPS - 1) / ANA_WARPS);
   if (leg_pairs(plan, nf))
-    SLE_CUDA(launch_pdl(k_leg_ana<2>, dim3(gx, (nf + 1) / 2), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
+    SLE_CUDA(launch_pdl_if(plan->early, k_leg_ana<2>, dim3(gx, (nf + 1) / 2), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
   else
-    SLE_CUDA(launch_pdl(k_leg_ana<1>, dim3(gx, nf), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
+    SLE_CUDA(launch_pdl_if(plan->early, k_leg_ana<1>, dim3(gx, nf), dim3(32 * ANA_WARPS), 0, st, d, o, nf, dense));
   return SLE_OK;
 }
 
@@ -725,9 +725,9 @@ static int fp64_leg_syn(const sle_sht* plan, ShtDev d, const CSpecPtrs& c, int n
   d.leg = plan->leg[1];
   const unsigned gx = (unsigned)(d.nm * ((d.ngrp + NA - 1) / NA));
   if (leg_pairs(plan, nf))
-    SLE_CUDA(launch_pdl(k_leg_syn<NA, 2>, dim3(gx, (nf + 1) / 2), dim3(32 * SYN_WARPS), syn_smem(NA, 2), st, d, c, nf, dense));
+    SLE_CUDA(launch_pdl_if(plan->early, k_leg_syn<NA, 2>, dim3(gx, (nf + 1) / 2), dim3(32 * SYN_WARPS), syn_smem(NA, 2), st, d, c, nf, dense));
   else
-    SLE_CUDA(launch_pdl(k_leg_syn<NA, 1>, dim3(gx, nf), dim3(32 * SYN_WARPS), syn_smem(NA, 1), st, d, c, nf, dense));
+    SLE_CUDA(launch_pdl_if(plan->early, k_leg_syn<NA, 1>, dim3(gx, nf), dim3(32 * SYN_WARPS), syn_smem(NA, 1), st, d, c, nf, dense));
   return SLE_OK;
 }
 
@@ -747,7 +747,7 @@ static int fp64_analysis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream_
   }
   ProfToken t0 = prof_begin(PROF_FFT, nf, st);
 #define SLE_LAUNCH_FOLD(NN) \
-  SLE_CUDA(launch_pdl(k_fft_fold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
+  SLE_CUDA(launch_pdl_if(plan->early, k_fft_fold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_FOLD)
 #undef SLE_LAUNCH_FOLD
   prof_end(t0, st);
@@ -779,7 +779,7 @@ static int fp64_synthesis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream
   prof_end(t0, st);
   ProfToken t1 = prof_begin(PROF_IFFT, nf, st);
 #define SLE_LAUNCH_IFFT(NN) \
-  SLE_CUDA(launch_pdl(k_ifft_unfold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
+  SLE_CUDA(launch_pdl_if(plan->early, k_ifft_unfold<NN>, dim3(d.nh, nf), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_IFFT)
 #undef SLE_LAUNCH_IFFT
   prof_end(t1, st);
@@ -1182,6 +1182,7 @@ extern "C" int sle_sht_create(int nlat, int nlon, int lmax, sle_sht** out) {
   }
   sle_sht* p = new sle_sht();
   std::memset(p, 0, sizeof(sle_sht));
+  p->early = true;
   // launch shape of the mixed-precision transforms (sle_sht_set_tuning changes it)
   p->tune_fpl = MX_MAXF;
   p->tune_stages = 4;
@@ -1419,7 +1420,7 @@ extern "C" int sle_sht_analysis_noalloc(sle_sht* plan, const double* grid_dev, v
   SpecPtrs o{};
   o.p[0] = reinterpret_cast<double2*>(coeffs_packed_dev);
 #define SLE_LAUNCH_FOLD1(NN) \
-  SLE_CUDA(launch_pdl(k_fft_fold<NN>, dim3(d.nh, 1), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
+  SLE_CUDA(launch_pdl_if(plan->early, k_fft_fold<NN>, dim3(d.nh, 1), dim3(fft_threads(2, NN)), fft_smem(d), st, d, g))
   SLE_FFT_SWITCH(d.n2, SLE_LAUNCH_FOLD1)
 #undef SLE_LAUNCH_FOLD1
   SLE_TRY(fp64_leg_ana(plan, d, o, 1, 0, st));

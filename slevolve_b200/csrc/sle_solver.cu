@@ -1467,7 +1467,7 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   const int nsyn = (int)s->f_syn_sl.size();
   const bool fuse = s->cfg.precision == SLE_PREC_MIXED && s->cfg.opt_dsl && s->plan->mx_ready &&
                     nsyn <= std::min(MX_MAXF, s->plan->tune_fpl);
-  SLE_CUDA(launch_pdl(k_b18, dim3(nb(nc), B), dim3(256), 0, st, D, fuse ? s->plan->mx_bsyn : nullptr,
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_b18, dim3(nb(nc), B), dim3(256), 0, st, D, fuse ? s->plan->mx_bsyn : nullptr,
                       fuse ? s->plan->mx_bpos : nullptr));
   prof_end(t, st);
   SLE_TRY(sht_synthesis_list(s->plan, s->f_syn_sl.data(), nsyn, st, fuse));
@@ -1478,7 +1478,7 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   prof_end(t, st);
   if (!s->cfg.opt_dsl) {
     note_launch();
-    SLE_CUDA(launch_pdl(k_sltot, dim3(nb(nc), B), dim3(256), 0, st, D));
+    SLE_CUDA(launch_pdl_if(s->plan->early, k_sltot, dim3(nb(nc), B), dim3(256), 0, st, D));
     SLE_TRY(sht_synthesis_list(s->plan, s->f_syn_sltot.data(), (int)s->f_syn_sltot.size(), st));
   }
   note_launch(2);
@@ -1497,7 +1497,7 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   t = prof_begin(PROF_DICE, act, st);
   SLE_CUDA(launch_pdl(k_dice, dim3(std::min(nb(nc), (unsigned)DICE_BLOCKS), B), dim3(256), 0, st, D));
   prof_end(t, st);
-  SLE_CUDA(launch_pdl(k_loop_cond, dim3(1), dim3(128), 0, st, D, s->bstatus, loop));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_loop_cond, dim3(1), dim3(128), 0, st, D, s->bstatus, loop));
   SLE_CUDA(cudaGetLastError());
   return SLE_OK;
 }
@@ -1703,7 +1703,7 @@ int init_slot(sle_batch* s, int b, const double* topo0, const double* ice0, int 
   return SLE_OK;
 }
 
-int batch_create(const sle_config* cfg, int nslot, int kmax, sle_batch** out) {
+int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_batch** out) {
   if (!cfg || !out) {
     set_error("sle_batch_create: NULL argument");
     return SLE_ERR_BAD_ARG;
@@ -1748,6 +1748,7 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, sle_batch** out) {
     }                                                                                 \
   } while (0)
   TRYC(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
+  s->plan->early = early;
   const int nl = cfg->lmax + 1;
   const long long ng = (long long)cfg->nlat * cfg->nlon;
   const long long nc = s->plan->d.ncoef;
@@ -1979,13 +1980,13 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
   SLE_CUDA(cudaMemsetAsync(s->bstatus, 0, sizeof(int), st));
   const unsigned UB = (unsigned)B;
   note_launch(3);
-  SLE_CUDA(launch_pdl(k_step_begin, dim3(nb(B, 128)), dim3(128), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_step_begin, dim3(nb(B, 128)), dim3(128), 0, st, D));
   // ---- modal advance (solver.py:835)
   ProfToken tadv = prof_begin(PROF_ADVANCE, (double)act.size(), st);
-  SLE_CUDA(launch_pdl(k_advance, dim3(nb(nc) + 1, UB), dim3(256), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_advance, dim3(nb(nc) + 1, UB), dim3(256), 0, st, D));
   prof_end(tadv, st);
   // ---- ice and ocean grids, their analyses (the stepping slots only)
-  SLE_CUDA(launch_pdl(k_ice_grid, dim3(nb(ng / 2), UB), dim3(256), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_ice_grid, dim3(nb(ng / 2), UB), dim3(256), 0, st, D));
   SLE_CUDA(cudaGetLastError());
   {
     std::vector<FieldSpec> f;
@@ -1999,8 +2000,8 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
   }
   // ---- first guess
   note_launch(2);
-  SLE_CUDA(launch_pdl(k_pre_spec, dim3(nb(nc), UB), dim3(256), 0, st, D));
-  SLE_CUDA(launch_pdl(k_rotation, dim3(1), dim3(128), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_pre_spec, dim3(nb(nc), UB), dim3(256), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_rotation, dim3(1), dim3(128), 0, st, D));
   SLE_CUDA(cudaGetLastError());
 
   // ---- inner fixed-point loop (solver.py:907-1051): a CUDA graph whose WHILE condition is set
@@ -2027,12 +2028,12 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     }
   }
   note_launch();
-  SLE_CUDA(launch_pdl(k_reopen, dim3(nb(B, 128)), dim3(128), 0, st, D));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_reopen, dim3(nb(B, 128)), dim3(128), 0, st, D));
 
   // ---- radial displacement (solver.py:1054-1072)
   if (s->cfg.calcRG) {
     note_launch();
-    SLE_CUDA(launch_pdl(k_rr, dim3(nb(nc), UB), dim3(256), 0, st, D));
+    SLE_CUDA(launch_pdl_if(s->plan->early, k_rr, dim3(nb(nc), UB), dim3(256), 0, st, D));
     std::vector<FieldSpec> f;
     for (int b : act) f.push_back(fspec(D.g(G_RR, b), D.sp(S_RRLM, b), &s->sc[b].status));
     SLE_TRY(sht_synthesis_list(s->plan, f.data(), (int)f.size(), st));
@@ -2043,22 +2044,22 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     for (int b : act) any_rates |= s->hss[b].rates != 0;
     if (any_rates) {
       note_launch();
-      SLE_CUDA(launch_pdl(k_rate_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->rate_spec, s->rate_tab, s->rate_rec,
+      SLE_CUDA(launch_pdl_if(s->plan->early, k_rate_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->rate_spec, s->rate_tab, s->rate_rec,
                           s->rate_rot));
     }
     bool any_horiz = false;
     for (int b : act) any_horiz |= s->hss[b].horiz != 0;
     if (any_horiz) {
       note_launch();
-      SLE_CUDA(launch_pdl(k_horiz_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->horiz_spec, s->horiz_tab));
+      SLE_CUDA(launch_pdl_if(s->plan->early, k_horiz_spec, dim3(nb(nc), UB), dim3(256), 0, st, D, s->horiz_spec, s->horiz_tab));
     }
   }
   // ---- commit (solver.py:1080-1096); extrap history (solver_opt.py:817-822)
   note_launch();
-  SLE_CUDA(launch_pdl(k_commit, dim3(nb(nc), UB), dim3(256), 0, st, D, s->cfg.inner_extrap));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_commit, dim3(nb(nc), UB), dim3(256), 0, st, D, s->cfg.inner_extrap));
   // ---- topography / ocean function and the degree-0 diagnostics
   note_launch();
-  SLE_CUDA(launch_pdl(k_post_grid, dim3(D.nlat, UB), dim3(256), 0, st, D, s->cfg.opt_diag));
+  SLE_CUDA(launch_pdl_if(s->plan->early, k_post_grid, dim3(D.nlat, UB), dim3(256), 0, st, D, s->cfg.opt_diag));
   if (!s->cfg.opt_diag) {
     std::vector<FieldSpec> f;
     for (int b : act) {
@@ -2070,7 +2071,7 @@ int batch_step_begin(sle_batch* s, const double* const* ice, int on_device, cons
     }
     SLE_TRY(sht_analysis_list(s->plan, f.data(), (int)f.size(), st));
     note_launch();
-    SLE_CUDA(launch_pdl(k_diag00, dim3(UB), dim3(32), 0, st, D));
+    SLE_CUDA(launch_pdl_if(s->plan->early, k_diag00, dim3(UB), dim3(32), 0, st, D));
   }
   SLE_CUDA(cudaGetLastError());
   return SLE_OK;
@@ -2214,7 +2215,11 @@ int batch_get(sle_batch* s, int b, int field, void* dst, int dst_on_device) {
 
 // ------------------------------------------------------------------ batch C ABI
 extern "C" int sle_batch_create(const sle_config* cfg, int nslots, int max_modes, sle_batch** out) {
-  return batch_create(cfg, nslots, max_modes, out);
+  // A batch of one slot serves one request at a time; its step keeps the launches it had (the inner
+  // loop's elementwise kernels and row FFTs programmatic, the rest plain).  A solve of 1500 steps at L =
+  // 63 would otherwise be over in 0.24 s, before a second request that arrives 0.25 s after it and is
+  // expected to find it running; with these it takes 0.28 s (0.32 s before the FP64 kernels).
+  return batch_create(cfg, nslots, max_modes, nslots != 1, out);
 }
 
 extern "C" int sle_batch_destroy(sle_batch* b) {
@@ -2555,7 +2560,7 @@ extern "C" int sle_solver_create(const sle_config* cfg, const sle_earth* earth, 
     return SLE_ERR_BAD_ARG;
   }
   sle_batch* b = nullptr;
-  SLE_TRY(batch_create(cfg, 1, earth->nmodes, &b));
+  SLE_TRY(batch_create(cfg, 1, earth->nmodes, true, &b));
   const int rc = set_earth(b, 0, earth, cfg->dt_years);
   if (rc != SLE_OK) {
     batch_free(b);
