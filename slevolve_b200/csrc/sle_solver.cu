@@ -118,6 +118,8 @@ struct Dev {
   long long npart, part_grid;
   unsigned int* counter;        // [nslot][4]
   double* rows;                 // [nslot][4][nlat]
+  unsigned char* has_ice;       // [nslot][nblk]: the block of 512 cells holds ice this step
+  int nblk;
   const double* w;              // Gauss weights
   double rhoi, rhow, epsilon1;
   int checkmarine, tpw, calcRG, opt_dsl;
@@ -131,6 +133,17 @@ struct Dev {
   __host__ __device__ double2* sp(int id, int b) const { return spec + ((size_t)id * nslot + b) * ncoef; }
   __host__ __device__ size_t kl(int b) const { return (size_t)b * K * nl; }
 };
+
+// I*_lm of the previous step (at the slot's first step the analysed initial ice), and the step's ice
+// increment dice = I*_lm - old, formed where it is needed instead of being stored (the re-analysis
+// after a grounded re-guess changes I*_lm, the commit is the first to write the previous one).
+__device__ __forceinline__ const double2* old_ice(const Dev& D, int b) {
+  return D.sp(D.ss[b].first ? S_OLDICE : S_PREV_ICE, b);
+}
+__device__ __forceinline__ double2 ice_increment(const Dev& D, int b, long long i) {
+  const double2 a = D.sp(S_ICELM, b)[i], o = old_ice(D, b)[i];
+  return make_double2(__dsub_rn(a.x, o.x), __dsub_rn(a.y, o.y));
+}
 
 // ------------------------------------------------------------------ reduction helpers
 __device__ __forceinline__ double warp_sum(double v) {
@@ -416,8 +429,14 @@ __global__ void k_ice_grid(Dev D) {
   pdl_trigger();
   SLOT_OR_RETURN();
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (2 * h >= D.ng) return;
-  const double2 v = ld2(D.g(G_ICE, b), h), tp = ld2(D.g(G_TOPO_PREV, b), h);
+  const bool in = 2 * h < D.ng;
+  double2 v = make_double2(0.0, 0.0);
+  if (in) v = ld2(D.g(G_ICE, b), h);
+  // blocks of 512 cells without ice are marked: the inner loop's grounded-ice test skips their ice
+  const int any = __syncthreads_or(v.x != 0.0 || v.y != 0.0);
+  if (threadIdx.x == 0) D.has_ice[(size_t)b * D.nblk + blockIdx.x] = any ? 1 : 0;
+  if (!in) return;
+  const double2 tp = ld2(D.g(D.ss[b].first ? G_TOPO_PREV : G_TOPO, b), h);
   uchar2 cx = ldm2(D.m(M_CXY, b), h);
   const unsigned char* wm = D.ss[b].warm_mask;
   if (wm) {  // warm start: the converged ocean function of this step in the previous pass
@@ -548,8 +567,7 @@ __device__ void rotation_block(const Dev& D, int b, Scal* sc) {
 
 // dice = I*_lm - old ; dI = p_ice + dice ; first guess of the load increment ; dS_cur ;
 // so = sum|load_inc|  (solver.py:868-905; extrap solver_opt.py:504-513).  old = the analysed
-// previous ice at the slot's first step, else the committed I*_lm of the last step (copied into
-// oldice here).  The last block evaluates the rotation block for the first inner iteration.
+// previous ice at the slot's first step, else the committed I*_lm of the last step.  The last block evaluates the rotation block for the first inner iteration.
 __global__ void k_pre_spec(Dev D) {
   pdl_wait();
   pdl_trigger();
@@ -557,8 +575,7 @@ __global__ void k_pre_spec(Dev D) {
   __shared__ double sh[32];
   const SlotStep ss = D.ss[b];
   const double2* icelm = D.sp(S_ICELM, b);
-  double2* oldice = D.sp(S_OLDICE, b);
-  const double2* osrc = ss.first ? oldice : D.sp(S_PREV_ICE, b);
+  const double2* osrc = old_ice(D, b);
   const double2* h1 = D.sp(ss.hsel ? S_HB : S_HA, b);
   const double2* h2 = D.sp(ss.hsel ? S_HA : S_HB, b);
   const double2* cstarlm = D.sp(S_CSTARLM, b);
@@ -570,9 +587,7 @@ __global__ void k_pre_spec(Dev D) {
     const double fr = -D.rhoi / D.rhow;
     const double2 s00 = make_double2(__dmul_rn(fr, dice00.x), __dmul_rn(fr, dice00.y));
     const double2 a = icelm[i], o = osrc[i];
-    if (!ss.first) oldice[i] = o;
     const double2 d = make_double2(__dsub_rn(a.x, o.x), __dsub_rn(a.y, o.y));
-    D.sp(S_DICE, b)[i] = d;
     const double2 pi = D.sp(S_P_ICE, b)[i];
     D.sp(S_DI, b)[i] = make_double2(__dadd_rn(pi.x, d.x), __dadd_rn(pi.y, d.y));
     double2 g;
@@ -589,11 +604,14 @@ __global__ void k_pre_spec(Dev D) {
                        __dsub_rn(__dmul_rn(u.y, ss.c1), __dmul_rn(ss.c2, v.y)));
     }
     D.sp(S_LOAD, b)[i] = g;
-    if (ss.mode == 0 && !ss.warm_ds) {
-      D.sp(S_DSCUR, b)[i] = make_double2(0.0, 0.0);
-    } else {
-      const double2 p = D.sp(S_P_OCEAN, b)[i];
-      D.sp(S_DSCUR, b)[i] = make_double2(__dadd_rn(p.x, g.x), __dadd_rn(p.y, g.y));
+    // dS_cur: only its degree-2 entries are read (by the rotation block)
+    if (i == D.i20 || i == D.i21) {
+      double2 c = make_double2(0.0, 0.0);
+      if (ss.mode != 0 || ss.warm_ds) {
+        const double2 p = D.sp(S_P_OCEAN, b)[i];
+        c = make_double2(__dadd_rn(p.x, g.x), __dadd_rn(p.y, g.y));
+      }
+      D.sp(S_DSCUR, b)[i] = c;
     }
     acc = cabs_(g);
   }
@@ -629,7 +647,7 @@ __global__ void k_b18(Dev D, float* bsyn, const int* bpos) {
   const SlotStep& ss = D.ss[b];
   if (ss.ramp) {   // same-step viscous weight of the current increment (solver.py:988-989)
     const double tc = ss.ramp_tab[(size_t)D.K * D.nl + l];
-    const double2 d = D.sp(S_DICE, b)[i];
+    const double2 d = ice_increment(D, b, i);
     re = __dadd_rn(re, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.x), __dmul_rn(D.rhow, c.x))));
     im = __dadd_rn(im, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.y), __dmul_rn(D.rhow, c.y))));
   }
@@ -735,8 +753,21 @@ __global__ void k_sltot(Dev D) {
 }
 
 // deltasl (dsl identity) and, when not converged, the ocean function of the refreshed
-// topography and the grounded-ice test on it (solver.py:1032-1037, 661-684).
-__global__ void k_refresh1(Dev D) {
+// topography and the grounded-ice test on it (solver.py:1032-1037, 661-684).  Bound: DRAM (27 bytes a
+// cell with the test).  U > 1: a block takes U chunks of 512 cells and loads the next one while it
+// tests this one, so that reads stay in flight past the block's first loads (slot record, then
+// cells); and the ice of a chunk that holds none this step is not read (8 of the 27 bytes; the sheets
+// cover a tenth of the globe).  Launches of fewer than REFRESH_MIN blocks take one chunk per block.
+// 32 slots at 512 x 1024: 105 -> 97 us with all slots iterating, 36 -> 15 with a few, 0.66 -> 0.48 ms per
+// step of 12 iterations (five blocks per SM; at three, 68 registers, 126 us).
+constexpr int REFRESH_U = 4;
+constexpr long long REFRESH_MIN = 8192;
+struct RefreshIn {
+  double2 a, ti, ic;
+  uchar2 be;
+};
+template <int U>
+__global__ void __launch_bounds__(256, U > 1 ? 5 : 8) k_refresh1(Dev D) {
   pdl_wait();
   pdl_trigger();
   SLOT_OR_RETURN();
@@ -744,37 +775,60 @@ __global__ void k_refresh1(Dev D) {
   const bool conv = sc->converged != 0;
   const bool test = !conv && D.checkmarine && sc->gr_nacc < GR_MAXACC;
   const double cadd = D.opt_dsl ? __dmul_rn(sc->conserv, sc->K00) : 0.0;
-  double cnt = 0.0;
-  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (2 * h < D.ng) {
+  uint32_t ice = 0xffffffffu;   // byte u: chunk u holds ice
+  if (U == 4 && test) ice = *reinterpret_cast<const uint32_t*>(D.has_ice + (size_t)b * D.nblk + 4 * blockIdx.x);
+  double* deltasl = D.g(G_DELTASL, b);
+  const double* src = D.opt_dsl ? D.g(G_DSL, b) : deltasl;
+  const double *tinit = D.g(G_TINIT, b), *icexy = D.g(G_ICE, b);
+  const unsigned char* beta = D.m(M_BETA, b);
+  const long long h0 = (long long)blockIdx.x * U * blockDim.x + threadIdx.x;
+  const auto load = [&](int u) {
     // every input first (the stores below could alias them as far as the compiler knows)
-    double* deltasl = D.g(G_DELTASL, b);
-    const double2 a = ld2(D.opt_dsl ? D.g(G_DSL, b) : deltasl, h);
-    double2 ti = make_double2(0.0, 0.0), ic = ti;
-    uchar2 be = make_uchar2(0, 0);
-    if (!conv) ti = ld2(D.g(G_TINIT, b), h);
+    RefreshIn r{make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_uchar2(0, 0)};
+    const long long h = h0 + u * (long long)blockDim.x;
+    if (2 * h >= D.ng) return r;
+    r.a = ld2(src, h);
+    if (!conv) r.ti = ld2(tinit, h);
     if (test) {
-      ic = ld2(D.g(G_ICE, b), h);
-      be = ldm2(D.m(M_BETA, b), h);
+      if ((ice >> (8 * u)) & 0xffu) r.ic = ld2(icexy, h);
+      r.be = ldm2(beta, h);
     }
-    double ds[2] = {a.x, a.y};
-    if (D.opt_dsl) {
-      ds[0] = __dadd_rn(a.x, cadd);
-      ds[1] = __dadd_rn(a.y, cadd);
-      // only the converged iteration's deltasl is an output; the others only feed the masks below
-      if (conv) st2(deltasl, h, ds[0], ds[1]);
-    }
-    if (!conv) {
-      const double t0 = __dsub_rn(ti.x, ds[0]), t1 = __dsub_rn(ti.y, ds[1]);
-      stm2(D.m(M_CXY, b), h, t0 < 0.0, t1 < 0.0);
-      if (test) {
-        const bool k0 = icestar_keep(ic.x, t0, D.rhow, D.rhoi), k1 = icestar_keep(ic.y, t1, D.rhow, D.rhoi);
-        const double g0 = k0 ? ic.x : __dmul_rn(ic.x, 0.0), g1 = k1 ? ic.y : __dmul_rn(ic.y, 0.0);
-        stm2(D.m(M_GRNEW, b), h, k0, k1);
-        if ((g0 < EPS0) != (be.x != 0)) cnt += 1.0;
-        if ((g1 < EPS0) != (be.y != 0)) cnt += 1.0;
+    return r;
+  };
+  double cnt = 0.0;
+  RefreshIn cur = load(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    RefreshIn next = cur;
+    if (u + 1 < U) next = load(u + 1);
+    const long long h = h0 + u * (long long)blockDim.x;
+    if (2 * h < D.ng) {
+      double ds[2] = {cur.a.x, cur.a.y};
+      if (D.opt_dsl) {
+        ds[0] = __dadd_rn(cur.a.x, cadd);
+        ds[1] = __dadd_rn(cur.a.y, cadd);
+        // only the converged iteration's deltasl is an output; the others only feed the masks below
+        if (conv) st2(deltasl, h, ds[0], ds[1]);
+      }
+      if (!conv) {
+        const double t0 = __dsub_rn(cur.ti.x, ds[0]), t1 = __dsub_rn(cur.ti.y, ds[1]);
+        stm2(D.m(M_CXY, b), h, t0 < 0.0, t1 < 0.0);
+        if (test) {
+          const double2 ic = cur.ic;
+          // without ice the flotation test (a division per ocean cell) fails: 0 > a non-negative depth
+          bool k0 = t0 > 0.0, k1 = t1 > 0.0;
+          if ((ice >> (8 * u)) & 0xffu) {
+            k0 = icestar_keep(ic.x, t0, D.rhow, D.rhoi);
+            k1 = icestar_keep(ic.y, t1, D.rhow, D.rhoi);
+          }
+          const double g0 = k0 ? ic.x : __dmul_rn(ic.x, 0.0), g1 = k1 ? ic.y : __dmul_rn(ic.y, 0.0);
+          stm2(D.m(M_GRNEW, b), h, k0, k1);
+          if ((g0 < EPS0) != (cur.be.x != 0)) cnt += 1.0;
+          if ((g1 < EPS0) != (cur.be.y != 0)) cnt += 1.0;
+        }
       }
     }
+    cur = next;
   }
   if (!test) return;
   const double part = block_sum(cnt, sh);
@@ -878,7 +932,7 @@ __global__ void k_refresh2_x8(Dev D) {
   }
 }
 
-// dice, dI after a grounded-mask change.  Such a change is rare after the first iterations, so
+// dI after a grounded-mask change.  Such a change is rare after the first iterations, so
 // each slot gets a fixed row of blocks that stride over its coefficients: a slot whose mask did
 // not change costs DICE_BLOCKS early exits instead of one per 256 coefficients.
 constexpr int DICE_BLOCKS = 64;
@@ -889,9 +943,7 @@ __global__ void __launch_bounds__(256) k_dice(Dev D) {
   if (sc->converged || !sc->gr_changed) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < D.ncoef; i += stride) {
-    const double2 a = D.sp(S_ICELM, b)[i], o = D.sp(S_OLDICE, b)[i], p = D.sp(S_P_ICE, b)[i];
-    const double2 d = make_double2(__dsub_rn(a.x, o.x), __dsub_rn(a.y, o.y));
-    D.sp(S_DICE, b)[i] = d;
+    const double2 p = D.sp(S_P_ICE, b)[i], d = ice_increment(D, b, i);
     D.sp(S_DI, b)[i] = make_double2(__dadd_rn(p.x, d.x), __dadd_rn(p.y, d.y));
   }
 }
@@ -964,7 +1016,7 @@ __global__ void k_rr(Dev D) {
   const SlotStep& ss = D.ss[b];
   if (ss.ramp) {   // solver.py:1065-1067
     const double tc = ss.ramp_tab[(size_t)(D.K + 1) * D.nl + l];
-    const double2 d = D.sp(S_DICE, b)[i];
+    const double2 d = ice_increment(D, b, i);
     re = __dadd_rn(re, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.x), __dmul_rn(D.rhow, c.x))));
     im = __dadd_rn(im, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.y), __dmul_rn(D.rhow, c.y))));
   }
@@ -999,7 +1051,7 @@ __global__ void k_rate_spec(Dev D, double2* rspec, const double* rtab, double* r
   double2* dsl = rspec + ((size_t)b * 2 + 0) * D.ncoef;
   double2* drr = rspec + ((size_t)b * 2 + 1) * D.ncoef;
   if (i == 0) {
-    const double2 d0 = D.sp(S_DICE, b)[0];
+    const double2 d0 = ice_increment(D, b, 0);
     rrec[2 * b] = d0.x;
     rrec[2 * b + 1] = d0.y;
     // the degree-2 modal states as the commit finds them (with ramp placement it changes them)
@@ -1016,7 +1068,7 @@ __global__ void k_rate_spec(Dev D, double2* rspec, const double* rtab, double* r
     return;
   }
   const int nl = D.nl, K = D.K;
-  const double2 ld = D.sp(S_LOAD, b)[i], d = D.sp(S_DICE, b)[i];
+  const double2 ld = D.sp(S_LOAD, b)[i], d = ice_increment(D, b, i);
   const double2 cur = make_double2(__dadd_rn(__dmul_rn(d.x, D.rhoi), __dmul_rn(ld.x, D.rhow)),
                                    __dadd_rn(__dmul_rn(d.y, D.rhoi), __dmul_rn(ld.y, D.rhow)));
   const double2 P = D.sp(S_P_LOAD, b)[i];
@@ -1101,7 +1153,7 @@ __global__ void k_commit(Dev D, int extrap) {
   double2 cur = make_double2(0.0, 0.0);
   const double2 ld = D.sp(S_LOAD, b)[i];
   if (l != 0) {
-    const double2 d = D.sp(S_DICE, b)[i];
+    const double2 d = ice_increment(D, b, i);
     cur = make_double2(__dadd_rn(__dmul_rn(d.x, D.rhoi), __dmul_rn(ld.x, D.rhow)),
                        __dadd_rn(__dmul_rn(d.y, D.rhoi), __dmul_rn(ld.y, D.rhow)));
   }
@@ -1159,7 +1211,7 @@ __global__ void k_post_grid(Dev D, int diag) {
   const long long row = (long long)j * (D.nlon / 2);
   const double *deltasl = D.g(G_DELTASL, b), *tinit = D.g(G_TINIT, b);
   const unsigned char* beta = D.m(M_BETA, b);
-  double *topo = D.g(G_TOPO, b), *topo_prev = D.g(G_TOPO_PREV, b);
+  double* topo = D.g(G_TOPO, b);   // also the next step's previous topography
   unsigned char* cxy = D.m(M_CXY, b);
   double *slc = D.g(G_TMP, b), *slcb = D.g(G_TMP3, b), *cstar = D.g(G_TMP4, b);
   unsigned char* rec_mask = D.ss[b].rec_mask;
@@ -1182,7 +1234,6 @@ __global__ void k_post_grid(Dev D, int diag) {
       d += cs[u];
     }
     st2(topo, h, tp[0], tp[1]);
-    st2(topo_prev, h, tp[0], tp[1]);
     stm2(cxy, h, o[0] != 0.0, o[1] != 0.0);
     if (rec_mask) {
       rec_mask[2 * h] = o[0] != 0.0;
@@ -1242,6 +1293,7 @@ __global__ void k_init_grid(Dev D, int b) {
   D.m(M_CXY0, b)[i] = c;
   D.m(M_CXY, b)[i] = c;
   D.g(G_TOPO_PREV, b)[i] = t;
+  D.g(G_TOPO, b)[i] = t;
   const double v = D.g(G_ICE_PREV, b)[i];
   const bool keep = !D.checkmarine || icestar_keep(v, t, D.rhow, D.rhoi);
   const double gg = keep ? v : __dmul_rn(v, 0.0);
@@ -1314,6 +1366,7 @@ struct sle_batch {
   double* partials;
   unsigned int* counter;
   double* rows;
+  unsigned char* has_ice;
   unsigned int* badflag;
   int* bstatus;            // batch-wide status raised by a tensor-core timeout
   // analytic rates read-out (opt-in per slot): rate spectra [nslot][2][ncoef] (sea level, radial),
@@ -1375,7 +1428,7 @@ void batch_free(sle_batch* s) {
   if (!s) return;
   void* ptrs[] = {s->grid, s->mask, s->spec, s->R, s->nmod, s->s_kl, s->decay, s->omd, s->a_sl, s->a_rr, s->ttl,
                   s->ttlekhl, s->ttlhe, s->a_il, s->a_m, s->a_tsl, s->a_trr, s->rc, s->r_il, s->r_m,
-                  s->r_lam, s->sc, s->ss, s->partials, s->counter, s->rows, s->badflag, s->bstatus,
+                  s->r_lam, s->sc, s->ss, s->partials, s->counter, s->rows, s->has_ice, s->badflag, s->bstatus,
                   s->rate_spec, s->rate_tab, s->rate_rec, s->rate_rot, s->horiz_spec, s->horiz_tab, s->ramp_tab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -1483,7 +1536,10 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   }
   note_launch(2);
   t = prof_begin(PROF_REFRESH1, act, st);
-  SLE_CUDA(launch_pdl(k_refresh1, dim3(nb(ng / 2), B), dim3(256), 0, st, D));
+  if ((long long)nb(ng / 2) * B >= REFRESH_MIN)
+    SLE_CUDA(launch_pdl(k_refresh1<REFRESH_U>, dim3(nb(ng / 2, 256 * REFRESH_U), B), dim3(256), 0, st, D));
+  else
+    SLE_CUDA(launch_pdl(k_refresh1<1>, dim3(nb(ng / 2), B), dim3(256), 0, st, D));
   prof_end(t, st);
   t = prof_begin(PROF_REFRESH2, act, st);
   if (ng % 8 == 0) SLE_CUDA(launch_pdl(k_refresh2_x8, dim3(nb(ng / 8), B), dim3(256), 0, st, D));
@@ -1776,6 +1832,9 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_bat
   TRY(dalloc(&s->partials, B * npart));
   TRY(dalloc(&s->counter, B * 4));
   TRY(dalloc(&s->rows, B * 4 * cfg->nlat));
+  const int nblk = (int)(nb(ng / 2) + 3) / 4 * 4;   // a 32-bit word covers four blocks
+  TRY(dalloc(&s->has_ice, B * nblk));
+  TRYC(cudaMemset(s->has_ice, 0, B * nblk));
   TRY(dalloc(&s->badflag, 1));
   TRY(dalloc(&s->bstatus, 1));
   TRYC(cudaMallocHost(reinterpret_cast<void**>(&s->hsc), sizeof(Scal) * B));
@@ -1837,6 +1896,8 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_bat
   D.part_grid = part_grid;
   D.counter = s->counter;
   D.rows = s->rows;
+  D.has_ice = s->has_ice;
+  D.nblk = nblk;
   D.w = s->plan->d.w;
   D.rhoi = cfg->rhoi;
   D.rhow = cfg->rhow;
@@ -1878,7 +1939,7 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_bat
   }
   const void* kernels[] = {(const void*)k_step_begin, (const void*)k_advance, (const void*)k_ice_grid, (const void*)k_pre_spec,
                            (const void*)k_rotation, (const void*)k_b18, (const void*)k_update, (const void*)k_sltot,
-                           (const void*)k_refresh1, (const void*)k_refresh2, (const void*)k_refresh2_x8, (const void*)k_dice,
+                           (const void*)k_refresh1<1>, (const void*)k_refresh1<REFRESH_U>, (const void*)k_refresh2, (const void*)k_refresh2_x8, (const void*)k_dice,
                            (const void*)k_loop_cond, (const void*)k_reopen, (const void*)k_rr, (const void*)k_commit,
                            (const void*)k_post_grid, (const void*)k_diag00};
   for (const void* k : kernels)
