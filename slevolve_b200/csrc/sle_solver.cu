@@ -171,12 +171,11 @@ __device__ double block_sum(double v, double* sh) {
 // index order and returns true (in all its threads) with *total set; others return false.  Only
 // thread 0's writes (the partial) are fenced before the block's ticket: a thread whose other
 // global writes the last block reads must __threadfence() them itself before calling.
-__device__ bool last_block_total(double part, double* partials, unsigned int* counter, double* total,
-                                 double* sh) {
+// The block's partials [first, first + U) are already stored by thread 0, of n in all.
+__device__ bool last_block_sum(double* partials, int n, unsigned int* counter, double* total, double* sh) {
   __shared__ bool is_last;
   __syncthreads();
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = part;
     __threadfence();
     const unsigned int t = atomicAdd(counter, 1u);
     is_last = (t == gridDim.x - 1);
@@ -185,7 +184,7 @@ __device__ bool last_block_total(double part, double* partials, unsigned int* co
   if (!is_last) return false;
   __threadfence();
   double v = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v += ((volatile double*)partials)[i];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) v += ((volatile double*)partials)[i];
   v = block_sum(v, sh);
   if (threadIdx.x == 0) {
     *total = v;
@@ -193,6 +192,11 @@ __device__ bool last_block_total(double part, double* partials, unsigned int* co
   }
   __syncthreads();
   return true;
+}
+
+__device__ bool last_block_total(double part, double* partials, unsigned int* counter, double* total, double* sh) {
+  if (threadIdx.x == 0) partials[blockIdx.x] = part;
+  return last_block_sum(partials, (int)gridDim.x, counter, total, sh);
 }
 
 // true in all threads of the slot's last block to finish (after every block passed this point)
@@ -622,58 +626,90 @@ __global__ void k_pre_spec(Dev D) {
   }
 }
 
+// Spectral passes of the inner loop: a block takes U runs of 256 coefficients and loads the next run
+// while it works on this one.  U = SPEC_U in launches of at least SPEC_MIN runs: the reads stay in flight
+// past a block's first loads, and a slot that converged costs a quarter of the early exits (32 slots at
+// L = 511, 16416 runs: load update 74 -> 76 us with all slots iterating, 23 -> 16 with a few, the B18 update
+// 54 and 19 -> 12; 6908 -> 6850 us of a step).
+constexpr int SPEC_U = 4;
+constexpr long long SPEC_MIN = 8192;
+
 // Eq. B18 (solver.py:977-991) plus the degree-2 rotational term of the current iteration.  With
 // bsyn (mixed precision, the iteration's synthesis one launch), the result goes straight into
 // that launch's B operand as field b instead of the FP64 spectrum, of which only (0, 0) is kept
 // (the degree-0 term the unfold adds in FP64).
-__global__ void k_b18(Dev D, float* bsyn, const int* bpos) {
+struct B18In {
+  int l;
+  double2 a, p, c, v;
+};
+template <int U>
+__global__ void __launch_bounds__(256, U > 1 ? 5 : 8) k_b18(Dev D, float* bsyn, const int* bpos) {
   pdl_wait();
   pdl_trigger();
   SLOT_OR_RETURN();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= D.ncoef) return;
-  if (i == 0) {
-    sc->gr_changed = 0;  // the previous iteration's mask changes are consumed
-    sc->cs_changed = 0;
-  }
-  const int l = D.lidx[i];
-  const double2 a = D.sp(S_DI, b)[i], bb = D.sp(S_P_OCEAN, b)[i], c = D.sp(S_LOAD, b)[i];
-  const double2 v = D.sp(S_VISC, b)[i];
-  const double te = D.ttlekhl[(size_t)b * D.nl + l], t = D.ttl[(size_t)b * D.nl + l];
-  double re = __dadd_rn(__dadd_rn(__dmul_rn(a.x, D.rhoi), __dmul_rn(bb.x, D.rhow)), __dmul_rn(c.x, D.rhow));
-  double im = __dadd_rn(__dadd_rn(__dmul_rn(a.y, D.rhoi), __dmul_rn(bb.y, D.rhow)), __dmul_rn(c.y, D.rhow));
-  re = __dadd_rn(__dmul_rn(re, te), __dmul_rn(v.x, t));
-  im = __dadd_rn(__dmul_rn(im, te), __dmul_rn(v.y, t));
+  const double2 *dI = D.sp(S_DI, b), *po = D.sp(S_P_OCEAN, b), *ld = D.sp(S_LOAD, b), *vi = D.sp(S_VISC, b);
+  const long long i0 = (long long)blockIdx.x * U * blockDim.x + threadIdx.x;
+  const auto load = [&](int u) {
+    const long long i = i0 + u * (long long)blockDim.x;
+    B18In r{};
+    if (i < D.ncoef) r = B18In{D.lidx[i], dI[i], po[i], ld[i], vi[i]};
+    return r;
+  };
   const SlotStep& ss = D.ss[b];
-  if (ss.ramp) {   // same-step viscous weight of the current increment (solver.py:988-989)
-    const double tc = ss.ramp_tab[(size_t)D.K * D.nl + l];
-    const double2 d = ice_increment(D, b, i);
-    re = __dadd_rn(re, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.x), __dmul_rn(D.rhow, c.x))));
-    im = __dadd_rn(im, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.y), __dmul_rn(D.rhow, c.y))));
-  }
-  if (D.tpw) {
-    const int q = (i == D.i20) ? 0 : (i == D.i21) ? 1 : (i == D.i22) ? 2 : -1;
-    if (q >= 0) {
-      re = __dadd_rn(re, sc->dsl_rot[2 * q]);
-      im = __dadd_rn(im, sc->dsl_rot[2 * q + 1]);
+  B18In cur = load(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    B18In next = cur;
+    if (u + 1 < U) next = load(u + 1);
+    const long long i = i0 + u * (long long)blockDim.x;
+    if (i >= D.ncoef) return;
+    if (i == 0) {
+      sc->gr_changed = 0;  // the previous iteration's mask changes are consumed
+      sc->cs_changed = 0;
     }
-  }
-  if (bsyn) {
-    mx_bsyn_put(bsyn, __ldg(bpos + i), b, i == 0 ? make_double2(0.0, 0.0) : make_double2(re, im));
-    if (i == 0) D.sp(S_SL, b)[0] = make_double2(re, im);
-  } else {
-    D.sp(S_SL, b)[i] = make_double2(re, im);
+    const int l = cur.l;
+    const double2 a = cur.a, bb = cur.p, c = cur.c, v = cur.v;
+    const double te = D.ttlekhl[(size_t)b * D.nl + l], t = D.ttl[(size_t)b * D.nl + l];
+    double re = __dadd_rn(__dadd_rn(__dmul_rn(a.x, D.rhoi), __dmul_rn(bb.x, D.rhow)), __dmul_rn(c.x, D.rhow));
+    double im = __dadd_rn(__dadd_rn(__dmul_rn(a.y, D.rhoi), __dmul_rn(bb.y, D.rhow)), __dmul_rn(c.y, D.rhow));
+    re = __dadd_rn(__dmul_rn(re, te), __dmul_rn(v.x, t));
+    im = __dadd_rn(__dmul_rn(im, te), __dmul_rn(v.y, t));
+    if (ss.ramp) {   // same-step viscous weight of the current increment (solver.py:988-989)
+      const double tc = ss.ramp_tab[(size_t)D.K * D.nl + l];
+      const double2 d = ice_increment(D, b, i);
+      re = __dadd_rn(re, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.x), __dmul_rn(D.rhow, c.x))));
+      im = __dadd_rn(im, __dmul_rn(tc, __dadd_rn(__dmul_rn(D.rhoi, d.y), __dmul_rn(D.rhow, c.y))));
+    }
+    if (D.tpw) {
+      const int q = (i == D.i20) ? 0 : (i == D.i21) ? 1 : (i == D.i22) ? 2 : -1;
+      if (q >= 0) {
+        re = __dadd_rn(re, sc->dsl_rot[2 * q]);
+        im = __dadd_rn(im, sc->dsl_rot[2 * q + 1]);
+      }
+    }
+    if (bsyn) {
+      mx_bsyn_put(bsyn, __ldg(bpos + i), b, i == 0 ? make_double2(0.0, 0.0) : make_double2(re, im));
+      if (i == 0) D.sp(S_SL, b)[0] = make_double2(re, im);
+    } else {
+      D.sp(S_SL, b)[i] = make_double2(re, im);
+    }
+    cur = next;
   }
 }
 
 // conserv, the load update and xi (solver.py:1002-1030):
 //   new = ((-dSprev + rO) + C*_lm conserv) - tO ;  dS_cur = dSprev + new ;  sa = sum|new|
-// The slot's last block decides its convergence.  Each block first prefetches into L2 the four
-// input spectra of the block one resident wave further on in launch order.
-__global__ void k_update(Dev D) {
+// The slot's last block decides its convergence; the partial sums are one per run of 256 coefficients
+// whatever U is, so that xi does not depend on it.  With U = 1 each block first prefetches into L2 the
+// four input spectra of the block one resident wave further on in launch order.
+struct UpdateIn {
+  double2 p, r, c, t;
+};
+template <int U>
+__global__ void __launch_bounds__(256) k_update(Dev D) {
   pdl_wait();
   pdl_trigger();
-  {
+  if (U == 1) {
     int bx, by;
     if (threadIdx.x < 4 && block_ahead(D.upd_ahead, bx, by) && !D.sc[D.slot0 + by].done) {
       const int b2 = D.slot0 + by;
@@ -690,6 +726,14 @@ __global__ void k_update(Dev D) {
   const double2* cstarlm = D.sp(S_CSTARLM, b);
   const double2* tOlm = D.sp(S_TOLM, b);
   const double2* dI = D.sp(S_DI, b);
+  const long long i0 = (long long)blockIdx.x * U * blockDim.x + threadIdx.x;
+  const auto load = [&](int u) {
+    const long long i = i0 + u * (long long)blockDim.x;
+    UpdateIn r{};
+    if (i < D.ncoef) r = UpdateIn{dSprev[i], rOlm[i], cstarlm[i], tOlm[i]};
+    return r;
+  };
+  UpdateIn cur = load(0);
   // conserv = ((1 / C*_00) * (-(rhoi/rhow) dI_00 - rO_00 + tO_00)).real
   const double2 c00 = cstarlm[0];
   const double2 rinv = np_cdiv(make_double2(1.0, 0.0), c00);
@@ -698,24 +742,34 @@ __global__ void k_update(Dev D) {
   const double2 x = make_double2(__dadd_rn(__dsub_rn(__dmul_rn(fr, d00.x), r00.x), t00.x),
                                  __dadd_rn(__dsub_rn(__dmul_rn(fr, d00.y), r00.y), t00.y));
   const double conserv = __dsub_rn(__dmul_rn(rinv.x, x.x), __dmul_rn(rinv.y, x.y));
-  double acc = 0.0;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < D.ncoef) {
-    const double2 p = dSprev[i], r = rOlm[i], c = cstarlm[i], t = tOlm[i];
-    double nr = __dadd_rn(-p.x, r.x), ni = __dadd_rn(-p.y, r.y);
-    nr = __dadd_rn(nr, __dmul_rn(c.x, conserv));
-    ni = __dadd_rn(ni, __dmul_rn(c.y, conserv));
-    nr = __dsub_rn(nr, t.x);
-    ni = __dsub_rn(ni, t.y);
-    D.sp(S_LOAD, b)[i] = make_double2(nr, ni);
-    // dS_cur = dS_prev + new: the rotation block of the next iteration reads its degree-2 entries;
-    // the commit forms the whole of it from the converged increment (the same sum)
-    if (i == D.i20 || i == D.i21) D.sp(S_DSCUR, b)[i] = make_double2(__dadd_rn(p.x, nr), __dadd_rn(p.y, ni));
-    acc = hypot(nr, ni);
+  double* partials = D.partials + (size_t)b * D.npart;
+  const int nrun = (int)((D.ncoef + blockDim.x - 1) / blockDim.x);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    UpdateIn next = cur;
+    if (u + 1 < U) next = load(u + 1);
+    const long long i = i0 + u * (long long)blockDim.x;
+    double acc = 0.0;
+    if (i < D.ncoef) {
+      const double2 p = cur.p, r = cur.r, c = cur.c, t = cur.t;
+      double nr = __dadd_rn(-p.x, r.x), ni = __dadd_rn(-p.y, r.y);
+      nr = __dadd_rn(nr, __dmul_rn(c.x, conserv));
+      ni = __dadd_rn(ni, __dmul_rn(c.y, conserv));
+      nr = __dsub_rn(nr, t.x);
+      ni = __dsub_rn(ni, t.y);
+      D.sp(S_LOAD, b)[i] = make_double2(nr, ni);
+      // dS_cur = dS_prev + new: the rotation block of the next iteration reads its degree-2 entries;
+      // the commit forms the whole of it from the converged increment (the same sum)
+      if (i == D.i20 || i == D.i21) D.sp(S_DSCUR, b)[i] = make_double2(__dadd_rn(p.x, nr), __dadd_rn(p.y, ni));
+      acc = hypot(nr, ni);
+    }
+    const double part = block_sum(acc, sh);
+    const int run = (int)blockIdx.x * U + u;
+    if (threadIdx.x == 0 && run < nrun) partials[run] = part;
+    cur = next;
   }
-  const double part = block_sum(acc, sh);
   double sa;
-  if (last_block_total(part, D.partials + (size_t)b * D.npart, D.counter + 4 * b, &sa, sh)) {
+  if (last_block_sum(partials, nrun, D.counter + 4 * b, &sa, sh)) {
     if (threadIdx.x == 0) {
       const double so = sc->so;
       double xi;
@@ -1520,14 +1574,20 @@ int enqueue_iteration(sle_batch* s, cudaGraphConditionalHandle loop) {
   const int nsyn = (int)s->f_syn_sl.size();
   const bool fuse = s->cfg.precision == SLE_PREC_MIXED && s->cfg.opt_dsl && s->plan->mx_ready &&
                     nsyn <= std::min(MX_MAXF, s->plan->tune_fpl);
-  SLE_CUDA(launch_pdl_if(s->plan->early, k_b18, dim3(nb(nc), B), dim3(256), 0, st, D, fuse ? s->plan->mx_bsyn : nullptr,
-                      fuse ? s->plan->mx_bpos : nullptr));
+  const bool runs = (long long)nb(nc) * B >= SPEC_MIN;
+  float* bsyn = fuse ? s->plan->mx_bsyn : nullptr;
+  const int* bpos = fuse ? s->plan->mx_bpos : nullptr;
+  if (runs)
+    SLE_CUDA(launch_pdl_if(s->plan->early, k_b18<SPEC_U>, dim3(nb(nc, 256 * SPEC_U), B), dim3(256), 0, st, D, bsyn, bpos));
+  else
+    SLE_CUDA(launch_pdl_if(s->plan->early, k_b18<1>, dim3(nb(nc), B), dim3(256), 0, st, D, bsyn, bpos));
   prof_end(t, st);
   SLE_TRY(sht_synthesis_list(s->plan, s->f_syn_sl.data(), nsyn, st, fuse));
   SLE_TRY(sht_analysis_list(s->plan, s->f_ana_ro.data(), (int)s->f_ana_ro.size(), st, PROF_ANA_STEP));
   note_launch();
   t = prof_begin(PROF_UPDATE, act, st);
-  SLE_CUDA(launch_pdl(k_update, dim3(nb(nc), B), dim3(256), 0, st, D));
+  if (runs) SLE_CUDA(launch_pdl(k_update<SPEC_U>, dim3(nb(nc, 256 * SPEC_U), B), dim3(256), 0, st, D));
+  else SLE_CUDA(launch_pdl(k_update<1>, dim3(nb(nc), B), dim3(256), 0, st, D));
   prof_end(t, st);
   if (!s->cfg.opt_dsl) {
     note_launch();
@@ -1869,7 +1929,7 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_bat
     TRYC(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     TRYC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_advance, 256, 0));
     D.adv_ahead = per_sm * nsm;
-    TRYC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_update, 256, 0));
+    TRYC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_update<1>, 256, 0));
     D.upd_ahead = per_sm * nsm;
   }
   D.nmod = s->nmod;
@@ -1938,7 +1998,7 @@ int batch_create(const sle_config* cfg, int nslot, int kmax, bool early, sle_bat
     s->use_graph = !(e && e[0] == '1');
   }
   const void* kernels[] = {(const void*)k_step_begin, (const void*)k_advance, (const void*)k_ice_grid, (const void*)k_pre_spec,
-                           (const void*)k_rotation, (const void*)k_b18, (const void*)k_update, (const void*)k_sltot,
+                           (const void*)k_rotation, (const void*)k_b18<1>, (const void*)k_b18<SPEC_U>, (const void*)k_update<1>, (const void*)k_update<SPEC_U>, (const void*)k_sltot,
                            (const void*)k_refresh1<1>, (const void*)k_refresh1<REFRESH_U>, (const void*)k_refresh2, (const void*)k_refresh2_x8, (const void*)k_dice,
                            (const void*)k_loop_cond, (const void*)k_reopen, (const void*)k_rr, (const void*)k_commit,
                            (const void*)k_post_grid, (const void*)k_diag00};
