@@ -37,7 +37,12 @@ constexpr int SEG = 64;
 constexpr double SIG_THRESHOLD = 1.0e-35;
 // The legacy literal of spat2spec / spec2spat (SLEvolve sht.py:60-61), not sqrt(2).
 constexpr double SQRT2_LEGACY = 1.41421356;
-constexpr int MAXF = 4;   // fields per batched transform launch (FP64 path); per call with the dense layout
+constexpr int MAXF = 32;          // most fields per FP64 transform launch (a plan's own limit: fp64_group)
+constexpr int DENSE_MAXF = 4;    // fields per call with the dense layout
+// A plan's FP64 launches carry as many fields as fit 64 MiB of folded FFTs (and as much of Legendre
+// sums), at least 4 and at most MAXF: 15 at L = 511, 32 up to L = 255.  With four for every plan, lists of
+// small fields paid two launches and a drain per four: FIGURES_GROUP
+constexpr size_t FP64_GROUP_BYTES = (size_t)64 << 20;
 constexpr int MAX_CALL_FIELDS = 256;   // fields per transform call with the packed layout
 constexpr int MX_MAXF = 32;          // fields per mixed-precision transform launch
 constexpr int MX_NMAX = 2 * MX_MAXF; // B-operand rows (Re, Im per field)
@@ -144,8 +149,8 @@ struct ShtDev {
   const unsigned char* istart;// [nseg] first significant latitude group of the segment
   LegSet leg;                 // what a launch of the FP64 Legendre kernels walks
   const double2* tw;          // [n2] exp(-2 pi i t / nlon)
-  double2* X;                 // [MAXF][2][nm][nh] folded rFFT (S then D) of analysed grids
-  double2* EO;                // [MAXF][nh][nm][2] even/odd Legendre sums of synthesised fields
+  double2* X;                 // [fp64_group][2][nm][nh] folded rFFT (S then D) of analysed grids
+  double2* EO;                // [fp64_group][nh][nm][2] even/odd Legendre sums of synthesised fields
   // Per-field gates of a launch (device flags read at kernel entry): field f is skipped (its
   // outputs left as they are) when gset[f] && *gset[f] != 0, or gclr[f] && *gclr[f] == 0.
   const int* gset[MAXF];
@@ -259,9 +264,10 @@ struct sle_sht {
   sle::LegSet leg[2];         // FP64 Legendre kernels: the segments, and shorter pieces (may be the same)
   double2 *seeds, *tw, *X, *EO;
   unsigned char* istart;
-  double2* packbuf;           // [MAXF][ncoef] packed staging for dense-layout calls
+  double2* packbuf;           // [DENSE_MAXF][ncoef] packed staging for dense-layout calls
   double* skipped_frac;       // host value: fraction of (l, m, j) work skipped
   double work_frac;
+  int fp64_group;             // fields per FP64 transform launch
   int precision;              // SLE_PREC_FP64 or SLE_PREC_MIXED
   int* mx_status;             // device status word raised on a tensor-core timeout (may be null)
   // mixed-precision transform buffers (allocated on first use)
@@ -309,7 +315,7 @@ bool prof_enabled();
 ProfToken prof_begin(int cls, double units, cudaStream_t st);
 void prof_end(const ProfToken& t, cudaStream_t st);
 
-// Transforms of a list of fields (packed spectra), launched in groups of MAXF (FP64) or
+// Transforms of a list of fields (packed spectra), launched in groups of the plan's fp64_group (FP64) or
 // MX_MAXF (mixed) fields with the precision of the plan (sle_sht.cu).
 int sht_analysis_list(sle_sht* plan, const FieldSpec* f, int n, cudaStream_t st, int prof_cls = PROF_LEG_ANA);
 // b_ready (mixed precision, n <= the plan's fields per launch): field f's B operand was written by

@@ -731,7 +731,7 @@ static int fp64_leg_syn(const sle_sht* plan, ShtDev d, const CSpecPtrs& c, int n
   return SLE_OK;
 }
 
-// One FP64 launch group (1..MAXF fields, all packed or all dense).
+// One FP64 launch group (1..fp64_group fields, all packed or all dense).
 static int fp64_analysis(sle_sht* plan, const FieldSpec* fs, int nf, cudaStream_t st, int prof_cls) {
   ShtDev d = plan->d;
   GridPtrs g{};
@@ -808,7 +808,7 @@ static MxFieldArgs mx_args(const FieldSpec* fs, int nf) {
 int sht_analysis_list(sle_sht* plan, const FieldSpec* f, int n, cudaStream_t st, int prof_cls) {
   if (n < 1) return SLE_OK;
   const bool mx = plan->precision == SLE_PREC_MIXED;
-  const int group = mx ? plan->tune_fpl : MAXF;
+  const int group = mx ? plan->tune_fpl : plan->fp64_group;
   // equal groups (the tensor-core kernels' cost depends on the launch, not on its width)
   const int ngroups = (n + group - 1) / group;
   for (int g = 0; g < ngroups; ++g) {
@@ -825,7 +825,7 @@ int sht_analysis_list(sle_sht* plan, const FieldSpec* f, int n, cudaStream_t st,
 int sht_synthesis_list(sle_sht* plan, const FieldSpec* f, int n, cudaStream_t st, bool b_ready) {
   if (n < 1) return SLE_OK;
   const bool mx = plan->precision == SLE_PREC_MIXED;
-  const int group = mx ? plan->tune_fpl : MAXF;
+  const int group = mx ? plan->tune_fpl : plan->fp64_group;
   const int ngroups = (n + group - 1) / group;
   for (int g = 0; g < ngroups; ++g) {
     const int lo = (int)((long long)n * g / ngroups), hi = (int)((long long)n * (g + 1) / ngroups);
@@ -1008,9 +1008,13 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   SLE_TRY(dalloc(&p->cf, d.ncoef));
   SLE_TRY(dalloc(&p->istart, d.nseg));
   SLE_TRY(dalloc(&p->tw, tw_table_len(d.n2)));
-  SLE_TRY(dalloc(&p->X, (size_t)MAXF * 2 * d.nm * d.nh));
-  SLE_TRY(dalloc(&p->EO, (size_t)MAXF * 2 * d.nm * d.nh));
-  SLE_TRY(dalloc(&p->packbuf, (size_t)MAXF * d.ncoef));
+  {
+    const size_t per = (size_t)2 * d.nm * d.nh;
+    p->fp64_group = (int)std::min<size_t>(MAXF, std::max<size_t>(4, FP64_GROUP_BYTES / (per * sizeof(double2))));
+    SLE_TRY(dalloc(&p->X, p->fp64_group * per));
+    SLE_TRY(dalloc(&p->EO, p->fp64_group * per));
+  }
+  SLE_TRY(dalloc(&p->packbuf, (size_t)DENSE_MAXF * d.ncoef));
   double* segmax = nullptr;
   int* fail = nullptr;
   SLE_TRY(dalloc(&segmax, (size_t)d.nseg * d.ngrp));
@@ -1253,7 +1257,7 @@ extern "C" int sle_sht_analysis(sle_sht* plan, int nfields, const double* const*
     set_error("sle_sht_analysis: NULL argument");
     return SLE_ERR_BAD_ARG;
   }
-  const int maxf = (layout == SLE_LAYOUT_PACKED) ? MAX_CALL_FIELDS : MAXF;
+  const int maxf = (layout == SLE_LAYOUT_PACKED) ? MAX_CALL_FIELDS : DENSE_MAXF;
   if (nfields < 1 || nfields > maxf) {
     set_error("sle_sht_analysis: nfields must be 1..%d for this layout", maxf);
     return SLE_ERR_BAD_ARG;
@@ -1286,7 +1290,7 @@ extern "C" int sle_sht_synthesis(sle_sht* plan, int nfields, const void* const* 
     set_error("sle_sht_synthesis: NULL argument");
     return SLE_ERR_BAD_ARG;
   }
-  const int maxf = (layout == SLE_LAYOUT_PACKED) ? MAX_CALL_FIELDS : MAXF;
+  const int maxf = (layout == SLE_LAYOUT_PACKED) ? MAX_CALL_FIELDS : DENSE_MAXF;
   if (nfields < 1 || nfields > maxf) {
     set_error("sle_sht_synthesis: nfields must be 1..%d for this layout", maxf);
     return SLE_ERR_BAD_ARG;

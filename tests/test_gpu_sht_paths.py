@@ -77,3 +77,27 @@ def test_paired_fields_equal_single_fields(n, nlon, L, nf):
         assert torch.equal(one, c[f])
         s.synthesis_device([one], [gone], layout=_lib.LAYOUT_PACKED)
         assert torch.equal(gone, back[f])
+
+
+@pytest.mark.parametrize("n,nlon,L,nf", [(64, 128, 63, 33), (64, 128, 63, 32), (180, 512, 170, 21), (512, 1024, 511, 16)])
+def test_long_lists_equal_single_fields(n, nlon, L, nf):
+    """Lists of a whole launch, one field more, and beyond the plan's limit: the same bits as alone."""
+    import torch
+
+    from slevolve_b200 import _lib, make_sht
+
+    s = make_sht("cuda", n, nlon, L)
+    gen = torch.Generator(device="cuda").manual_seed(nf)
+    g = [torch.randn((n, nlon), dtype=torch.float64, device="cuda", generator=gen) for _ in range(nf)]
+    c = [torch.full((s.ncoef,), float("nan"), dtype=torch.complex128, device="cuda") for _ in g]
+    back = [torch.full_like(x, float("nan")) for x in g]
+    s.analysis_device(g, c, layout=_lib.LAYOUT_PACKED)
+    s.synthesis_device(c, back, layout=_lib.LAYOUT_PACKED)
+    one, gone = torch.empty_like(c[0]), torch.empty_like(g[0])
+    for f in range(nf):
+        s.analysis_device([g[f]], [one], layout=_lib.LAYOUT_PACKED)
+        assert torch.equal(one, c[f]), f
+        s.synthesis_device([one], [gone], layout=_lib.LAYOUT_PACKED)
+        assert torch.equal(gone, back[f]), f
+    with pytest.raises(ValueError):   # the dense layout's limit is unchanged
+        s.analysis_device(g[:5], [torch.empty((L + 1, L + 1), dtype=torch.complex128, device="cuda") for _ in range(5)])
