@@ -877,8 +877,8 @@ static void plan_free(sle_sht* p) {
   if (p->leg[1].fsegoff != p->leg[0].fsegoff) leg_set_free(p->leg[1], p->seeds);
   leg_set_free(p->leg[0], p->seeds);
   void* ptrs[] = {p->mu, p->w, p->wn, p->ws, p->be, p->cf, p->moff, p->lidx, p->segoff,
-                  p->seg_m, p->seg_l0, p->seeds, p->tw, p->X, p->EO, p->istart,
-                  p->packbuf, p->mx_xf, p->mx_twf, p->mx_gns, p->mx_bsyn, p->mx_s0, p->mx_abort,
+                  p->seg_m, p->seg_l0, p->seeds, p->tw, p->X, p->istart,
+                  p->mx_xf, p->mx_twf, p->mx_gns, p->mx_bsyn, p->mx_s0, p->mx_abort,
                   p->mx_ana_units, p->mx_syn_units, p->mx_syn_seg, p->mx_tab_ana, p->mx_tab_syn,
                   p->mx_ana_cta, p->mx_syn_cta, p->mx_bpos};
   for (void* q : ptrs)
@@ -1009,12 +1009,14 @@ static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
   SLE_TRY(dalloc(&p->istart, d.nseg));
   SLE_TRY(dalloc(&p->tw, tw_table_len(d.n2)));
   {
+    // X, EO and packbuf from one allocation: an allocation above 1 MB takes about 0.4 ms whatever its size
     const size_t per = (size_t)2 * d.nm * d.nh;
     p->fp64_group = (int)std::min<size_t>(MAXF, std::max<size_t>(4, FP64_GROUP_BYTES / (per * sizeof(double2))));
-    SLE_TRY(dalloc(&p->X, p->fp64_group * per));
-    SLE_TRY(dalloc(&p->EO, p->fp64_group * per));
+    const size_t nx = (p->fp64_group * per + 15) / 16 * 16;   // 256-byte boundaries
+    SLE_TRY(dalloc(&p->X, 2 * nx + (size_t)DENSE_MAXF * d.ncoef));
+    p->EO = p->X + nx;
+    p->packbuf = p->EO + nx;
   }
-  SLE_TRY(dalloc(&p->packbuf, (size_t)DENSE_MAXF * d.ncoef));
   double* segmax = nullptr;
   int* fail = nullptr;
   SLE_TRY(dalloc(&segmax, (size_t)d.nseg * d.ngrp));
