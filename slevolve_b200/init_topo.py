@@ -74,7 +74,7 @@ def relaxed_love(love, lmax, tau):
     h, k = np.array(love.he[:lmax + 1], float), np.array(love.ke[:lmax + 1], float)
     nl = lmax + 1
     nm = np.asarray(love.nmod[:nl], int)
-    K = int(nm[1:].max()) if nl > 1 else 0
+    K = min(int(nm[1:].max()), len(love.s)) if nl > 1 else 0
     if K == 0:
         return h, k
     on = np.arange(K)[:, None] < nm[None, :]   # the degree's modes
