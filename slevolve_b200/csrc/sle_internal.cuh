@@ -41,7 +41,7 @@ constexpr int MAXF = 32;         // most fields per FP64 transform launch (a pla
 constexpr int DENSE_MAXF = 4;    // fields per call with the dense layout
 // A plan's FP64 launches carry as many fields as fit 32 MiB of folded FFTs (and as much of Legendre
 // sums), at least 4 and at most MAXF: 7 at L = 511, 32 up to L = 255.  With four for every plan, lists of
-// small fields paid two launches and a drain per four: seven analyses at 180 x 512, L = 128, took
+// small fields paid two launches and a drain per four: seven analyses at 180 x 512, L = 170, took
 // 27.4 us with four per launch and take 18.1, 32 at 64 x 128 40.5 and 12.8.  A field of L = 511 fills
 // the chip by itself, and the byte limit keeps such a plan's scratch in the L2.
 constexpr size_t FP64_GROUP_BYTES = (size_t)32 << 20;
