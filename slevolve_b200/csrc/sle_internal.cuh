@@ -119,6 +119,14 @@ inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t sme
 // fewer blocks fit).  FP64 step at L = 511 773 -> 734 us, 32-member batch step 7290 -> 7160 us.
 constexpr int SMEM_CARVEOUT = 44;
 
+// Work item of the FP64 Legendre synthesis: an order, a latitude tile, and two masks over the order's
+// pieces, bit k for piece k: those significant on the whole tile, and those significant on its upper
+// half only.  64 bits: order 0 has 33 pieces at the largest degree, 2048.
+struct SynItem {
+  int m, tile;
+  unsigned long long full, half;
+};
+
 // What the FP64 Legendre kernels walk: pieces of fseg degrees (a segment or an even fraction of one),
 // their seeds, the first piece of each order, and the work items.
 struct LegSet {
@@ -126,10 +134,9 @@ struct LegSet {
   const double2* fseeds;      // [nfseg][nh], in the segment's scale
   const int* fsegoff;         // [nm+1]
   // analysis: (piece, order, first degree, first significant latitude group), most work first;
-  // synthesis: (order, latitude tile, mask of the order's pieces significant on the whole tile, mask
-  // of those significant on its upper half only), most work first
+  // synthesis: most work first
   const int4* ana_items;      // [nfseg]
-  const int4* syn_items;      // [nm * tiles]
+  const SynItem* syn_items;   // [nm * tiles]
 };
 
 // Device view of a transform plan, passed to kernels by value.

@@ -567,14 +567,12 @@ __device__ __forceinline__ void syn_segment(const sle::ShtDev& P, int s, int j0,
   }
 }
 
-// Item of a block: order, latitude tile, and its significant segments as two bit masks over the
-// order's segments (all latitude groups of the tile; only the upper half of them).  Warp w takes
-// every fourth segment of the union from the w-th on.
+// Warp w of the item's block takes every fourth piece of the two masks' union from the w-th on.
 template <int NA, int F>
-__device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const double2* const (&Uf)[F], int f0,
+__device__ __forceinline__ void syn_block(const sle::ShtDev& P, const SynItem& item, const double2* const (&Uf)[F], int f0,
                                           bool dense, double* sm) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = item.x, hb = item.y;
+  const int m = item.m, hb = item.tile;
   double2* su = reinterpret_cast<double2*>(sm) + (size_t)w * SEG * F;                          // [SEG][F]
   double* sb = sm + (size_t)SYN_WARPS * SEG * F * 2 + (size_t)w * SEG;                         // [SEG]
   double2* part = reinterpret_cast<double2*>(sm + (size_t)SYN_WARPS * SEG * (2 * F + 1));      // partial sums
@@ -586,10 +584,10 @@ __device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const
   for (int f = 0; f < F; ++f)
 #pragma unroll
     for (int i = 0; i < NA; ++i) E[f][i] = O[f][i] = make_double2(0.0, 0.0);
-  uint32_t left = (uint32_t)(item.z | item.w);
+  unsigned long long left = item.full | item.half;
   for (int n = 0; left; ++n, left &= left - 1) {
     if ((n & (SYN_WARPS - 1)) != w) continue;
-    const int k = __ffs(left) - 1, s = seg0 + k, l0 = m + P.leg.fseg * k;
+    const int k = __ffsll((long long)left) - 1, s = seg0 + k, l0 = m + P.leg.fseg * k;
     const int len = min(P.leg.fseg, P.lmax + 1 - l0);
     const long long base = moff + P.leg.fseg * k;
     __syncwarp();
@@ -605,7 +603,7 @@ __device__ __forceinline__ void syn_block(const sle::ShtDev& P, int4 item, const
       sb[t] = in ? P.be[base + t] : 0.0;
     }
     __syncwarp();
-    if (NA > 1 && !(((uint32_t)item.z >> k) & 1u)) syn_segment<NA, NA / 2, F>(P, s, j0, len, su, sb, E, O);
+    if (NA > 1 && !((item.full >> k) & 1u)) syn_segment<NA, NA / 2, F>(P, s, j0, len, su, sb, E, O);
     else syn_segment<NA, 0, F>(P, s, j0, len, su, sb, E, O);
   }
   // partial sums [warp][field][latitude group][E | O][lane]
@@ -644,7 +642,7 @@ constexpr size_t syn_smem(int na, int f) {
 template <int NA, int F>
 __global__ void __launch_bounds__(32 * SYN_WARPS, F == 1 ? 4 : 3) k_leg_syn(sle::ShtDev P, CSpecPtrs in, int nf, int dense) {
   extern __shared__ double smd[];
-  const int4 item = P.leg.syn_items[blockIdx.x];
+  const SynItem item = P.leg.syn_items[blockIdx.x];
   pdl_wait();
   pdl_trigger();
   const int f0 = F * blockIdx.y;
@@ -924,13 +922,13 @@ static int leg_set_build(sle_sht* p, LegSet& set, int split, const std::vector<i
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return work[a] > work[b]; });
     return order;
   };
-  const auto upload = [](const std::vector<int4>& items, const std::vector<int>& order, const int4** out) -> int {
-    std::vector<int4> v;
-    for (int i : order) v.push_back(items[i]);
-    int4* dev = nullptr;
+  const auto upload = [](const auto& items, const std::vector<int>& order, auto** out) -> int {
+    auto v = items;
+    for (size_t i = 0; i < v.size(); ++i) v[i] = items[order[i]];
+    auto* dev = v.data();
     SLE_TRY(dalloc(&dev, v.size()));
     *out = dev;
-    SLE_CUDA(cudaMemcpy(dev, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    SLE_CUDA(cudaMemcpy(dev, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
     return SLE_OK;
   };
   std::vector<int4> items;
@@ -942,24 +940,28 @@ static int leg_set_build(sle_sht* p, LegSet& set, int split, const std::vector<i
   SLE_TRY(upload(items, by_work(work), &set.ana_items));
   // synthesis blocks: (order, latitude tile) with the tile's significant pieces
   const int na = syn_na(d), ntile = (d.ngrp + na - 1) / na;
-  items.clear();
+  std::vector<SynItem> tiles;
   work.clear();
   for (int m = 0; m < d.nm; ++m) {
+    if (foff[m + 1] - foff[m] > 64) {
+      set_error("order %d has %d pieces, more than its work items' masks hold", m, foff[m + 1] - foff[m]);
+      return SLE_ERR_BAD_SHAPE;
+    }
     for (int t = 0; t < ntile; ++t) {
       const int glo = na * t, ghi = std::min(glo + na, d.ngrp) - 1;
-      uint32_t full = 0, half = 0;
+      unsigned long long full = 0, half = 0;
       long long c = 0;
       for (int i = foff[m]; i < foff[m + 1]; ++i) {
         if (f_ist[i] > ghi) continue;
         const bool upper = na > 1 && f_ist[i] >= glo + na / 2;
-        (upper ? half : full) |= 1u << (i - foff[m]);
+        (upper ? half : full) |= 1ull << (i - foff[m]);
         c += (long long)std::min(set.fseg, L + 1 - f_l0[i]) * (upper ? 1 : 2);
       }
-      items.push_back(make_int4(m, t, (int)full, (int)half));
+      tiles.push_back(SynItem{m, t, full, half});
       work.push_back(c);
     }
   }
-  return upload(items, by_work(work), &set.syn_items);
+  return upload(tiles, by_work(work), &set.syn_items);
 }
 
 static int plan_build(sle_sht* p, int nlat, int nlon, int lmax) {
