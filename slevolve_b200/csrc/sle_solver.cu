@@ -2408,12 +2408,14 @@ int snap_flags(const sle_config& c) {
          (c.opt_diag ? 16 : 0) | (c.inner_extrap ? 32 : 0);
 }
 
-// The device sections of slot b: (device address, bytes), in image order.
-std::vector<std::pair<void*, size_t>> snap_sections(sle_batch* s, int b) {
+// The device sections of slot b: (device address, bytes), in image order.  The step keeps one copy of the
+// topography and reads G_TOPO_PREV in a slot's first step only; a saved image holds the topography in
+// both places, so that every library of this image version continues from it.
+std::vector<std::pair<void*, size_t>> snap_sections(sle_batch* s, int b, bool save) {
   const Dev& D = s->D;
   const size_t ng = (size_t)D.ng, nc = (size_t)D.ncoef, nl = (size_t)D.nl, K = (size_t)s->K;
   std::vector<std::pair<void*, size_t>> v;
-  for (int g = 0; g < NGRID; ++g) v.push_back({D.g(g, b), sizeof(double) * ng});
+  for (int g = 0; g < NGRID; ++g) v.push_back({D.g(save && g == G_TOPO_PREV ? G_TOPO : g, b), sizeof(double) * ng});
   for (int m = 0; m < NMASK; ++m) v.push_back({D.m(m, b), ng});
   for (int q = 0; q < NSPEC; ++q) v.push_back({D.sp(q, b), sizeof(double2) * nc});
   if (K) v.push_back({D.R + (size_t)b * K * nc, sizeof(double2) * K * nc});
@@ -2437,7 +2439,7 @@ std::vector<std::pair<void*, size_t>> snap_sections(sle_batch* s, int b) {
 
 long long snap_bytes(sle_batch* s) {
   long long n = (long long)sizeof(SnapHeader);
-  for (const auto& sec : snap_sections(s, 0)) n += (long long)sec.second;
+  for (const auto& sec : snap_sections(s, 0, true)) n += (long long)sec.second;
   return n;
 }
 
@@ -2478,7 +2480,7 @@ int batch_snapshot(sle_batch* s, int b, void* dst, long long nbytes) {
   unsigned char* out = static_cast<unsigned char*>(dst);
   std::memcpy(out, &hd, sizeof(hd));
   size_t off = sizeof(hd);
-  for (const auto& sec : snap_sections(s, b)) {
+  for (const auto& sec : snap_sections(s, b, true)) {
     SLE_CUDA(cudaMemcpyAsync(out + off, sec.first, sec.second, cudaMemcpyDeviceToHost, s->st));
     off += sec.second;
   }
@@ -2514,7 +2516,7 @@ int batch_restore(sle_batch* s, int b, const void* src, long long nbytes) {
   }
   const unsigned char* in = static_cast<const unsigned char*>(src);
   size_t off = sizeof(hd);
-  for (const auto& sec : snap_sections(s, b)) {
+  for (const auto& sec : snap_sections(s, b, false)) {
     SLE_CUDA(cudaMemcpyAsync(sec.first, in + off, sec.second, cudaMemcpyHostToDevice, s->st));
     off += sec.second;
   }
