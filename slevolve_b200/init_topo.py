@@ -73,8 +73,13 @@ def relaxed_love(love, lmax, tau):
     sum_k r_k / s_k (1 - exp(-s_k tau)) over the degree's modes (init_topo_segmented.py:114-118)."""
     h, k = np.array(love.he[:lmax + 1], float), np.array(love.ke[:lmax + 1], float)
     nl = lmax + 1
+    if nl <= 1:
+        return h, k
     nm = np.asarray(love.nmod[:nl], int)
-    K = min(int(nm[1:].max()), len(love.s)) if nl > 1 else 0
+    have = min(len(h), len(k), len(nm), *(np.shape(a)[1] for a in (love.s, love.r, love.rprime)))
+    if have < nl:
+        raise IndexError(f"the Earth model's tables hold degrees up to {have - 1}, not {lmax}")
+    K = min(int(nm[1:].max()), len(love.s))
     if K == 0:
         return h, k
     on = np.arange(K)[:, None] < nm[None, :]   # the degree's modes
