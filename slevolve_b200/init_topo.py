@@ -163,7 +163,7 @@ def segmented_guess(Tp, ice, love, lmax, dt, threshold=0.01, start=None, c0=62.0
     the reference's ``segmented_guess``."""
     import torch
 
-    from .sht import make_sht
+    from .sht import CudaSHT, make_sht
 
     def dev(x):
         if isinstance(x, torch.Tensor):
@@ -174,10 +174,10 @@ def segmented_guess(Tp, ice, love, lmax, dt, threshold=0.01, start=None, c0=62.0
     nl, no = Tp_d.shape
     N = len(ice) - 1
     sht = sht if sht is not None else make_sht("cuda", nl, no, lmax)
-    # the transform's own Gauss weights (leggauss solves an eigenvalue problem for them)
-    weights = getattr(sht, "weights", None)
-    g = _Grids(Tp_d, dev(ice[0]), dev(ice[N]), rhoi, rhow, radius, torch,
-               weights if weights is not None and len(weights) == nl else None)
+    # this package's transform holds the Gauss weights of its rows (leggauss solves an eigenvalue problem
+    # for them); what another transform calls its weights need not be these
+    own = type(sht) is CudaSHT and sht.nlat == nl
+    g = _Grids(Tp_d, dev(ice[0]), dev(ice[N]), rhoi, rhow, radius, torch, sht.weights if own else None)
     V = np.array([float((dev(ice[n]) * g.area).sum()) for n in range(N + 1)])
     segs = segments(V, dt, threshold)
     l = np.arange(lmax + 1, dtype=float)
