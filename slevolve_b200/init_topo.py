@@ -9,8 +9,9 @@ the sea-level change dSL = c + S is iterated to a fixed point (area-weighted RMS
 water-volume residual (init_topo_segmented.py:84-98, 101-146).
 
 Here the grids stay on the device: every G - R operator is one analysis and one synthesis of the
-FP64 CUDA transform (``make_sht("cuda")``), the bisection evaluates the residual with one fused
-reduction kernel per step (``sle_topo_residual``), and the elementwise updates run on the device.
+FP64 CUDA transform (``make_sht("cuda")``), the bisection runs on the device, four of its steps per
+launch of one fused reduction kernel (``sle_topo_bisect``; ``sle_topo_residual`` evaluates a single
+point), and the elementwise updates run there too.
 The leg detection works on the ice-volume series (N + 1 numbers) on the host, as do the relaxed
 Love numbers (a few hundred numbers per leg).
 """
@@ -110,9 +111,7 @@ class _Grids:
         self.Cp = (Tp < 0) & ~self.gp
         self.Cp_f = self.Cp.to(torch.float64)
         self.Vp = float(((-Tp).clamp(min=0) * self.Cp * self.area).sum())
-        self.scratch = torch.zeros(int(_lib.lib().sle_topo_scratch_bytes()), dtype=torch.uint8, device="cuda")
-        self.out2 = (C.c_double * 2)()
-        self.bisect_scratch = None
+        self.scratch = self.bisect_scratch = None
 
     def grounded(self, I, T):
         return (I > 0) & ((T > 0) | (self.rhoi * I > self.rhow * T.abs()))
@@ -126,13 +125,16 @@ class _Grids:
     def residual(self, S, c):
         """Water-volume residual of T0 = (Tp + c) + S (init_topo_segmented.py:84-90)."""
         nl, no = self.Tp.shape
+        if self.scratch is None:
+            self.scratch = self.t.zeros(int(_lib.lib().sle_topo_scratch_bytes()), dtype=self.t.uint8, device="cuda")
+        out2 = (C.c_double * 2)()
         st = self.t.cuda.current_stream().cuda_stream
         _lib.check(_lib.lib().sle_topo_residual(
             C.c_void_p(self.Tp.data_ptr()), C.c_void_p(S.data_ptr()), float(c), C.c_void_p(self.I0.data_ptr()),
             C.c_void_p(self.Ip.data_ptr()), C.c_void_p(self.gp_u8.data_ptr()), C.c_void_p(self.wrow.data_ptr()),
-            nl, no, self.rhoi, self.rhow, C.c_void_p(self.scratch.data_ptr()), self.out2, C.c_void_p(st)),
+            nl, no, self.rhoi, self.rhow, C.c_void_p(self.scratch.data_ptr()), out2, C.c_void_p(st)),
             "sle_topo_residual")
-        return self.out2[0] - self.Vp + self.rhoi / self.rhow * self.out2[1]
+        return out2[0] - self.Vp + self.rhoi / self.rhow * out2[1]
 
     def solve_c(self, S, c, half):
         """60 bisection steps of the residual over c +- half (init_topo_segmented.py:91-98), decided on
