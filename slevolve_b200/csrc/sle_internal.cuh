@@ -112,11 +112,16 @@ inline cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t sme
 }
 
 
-// Shared-memory share (percent of 228 KB: the 100 KB setting) that every kernel but the tensor-core ones
-// asks for.  Kernels that ask for different shares cannot share an SM, so that a kernel scheduled early
+// Shared-memory share (percent of 228 KB: the 100 KB setting) that the row FFTs, the FP64 Legendre
+// kernels, the synthesis B operand and the kernels of the step ask for (the tensor-core kernels take what
+// their shared memory needs; set-up, packing, read-outs and the segmented guess leave it to the driver).
+// Kernels that ask for different shares cannot share an SM, so that a kernel scheduled early
 // waits for the SM to drain and reconfigure; and the row FFTs read their twiddles through the L1 that
 // the rest leaves (32-field fold at L = 511: 69.4 us at 100 percent, 58.4 at 44, 84.4 at 28, where
 // fewer blocks fit).  FP64 step at L = 511 773 -> 734 us, 32-member batch step 7290 -> 7160 us.
+// Rows of 2048 and 4096 longitudes fit one or two blocks at this share where 100 percent fits more; whole
+// transforms there are still 1.15 to 2 times as fast as with the kernels and shares before (16 fields at
+// 512 x 4096, L = 511: analysis 571 -> 378 us, synthesis 535 -> 376).
 constexpr int SMEM_CARVEOUT = 44;
 
 // Work item of the FP64 Legendre synthesis: an order, a latitude tile, and two masks over the order's

@@ -1420,7 +1420,8 @@ int sht_mx_synthesis(sle_sht* p, const MxFieldArgs& a, int* status, cudaStream_t
 // The abort flag after the work enqueued on `st`: waits for the stream and reads the host copy (a
 // device-to-host copy of one word costs a transfer more per call).  As with such a copy on the legacy
 // default stream, a non-blocking stream is not waited for: the call returns at once and reports what
-// earlier, finished work raised.  While the stream is being captured the copy stays.
+// earlier, finished work raised.  While the stream is being captured the copy stays: capture
+// refuses it, as before (only a relaxed capture of a non-blocking stream lets it through).
 int sht_mx_abort_flag(sle_sht* p, int* flag, cudaStream_t st) {
   *flag = 0;
   if (!p->mx_ready) return SLE_OK;

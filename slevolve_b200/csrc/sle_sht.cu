@@ -341,8 +341,10 @@ __global__ void __launch_bounds__(fft_nt(2, N)) k_ifft_unfold(sle::ShtDev P, Out
 // through shared memory (each lane stores its 16 partial sums, a pair of lanes adds the 32 of one
 // value), which costs about 6 instructions per degree, where a butterfly with its selects and
 // two-word shuffles cost 27.  The totals collect in shared memory and leave scaled and coalesced.
-// Bound: the FP64 pipe (one warp instruction per 2.2 cycles and scheduler).  F = 2 shares one
-// recurrence between two fields (6 operations instead of 8 per degree and latitude).
+// Bound: FP64 issue while there are warps to issue from; a single field at L = 511 is bound by its
+// chains of dependent operations (FP64 pipe active in 42 % of the SMs' active cycles, ten warps per SM,
+// blocks for 1.3 waves).  F = 2 shares one recurrence between two fields (6 operations instead of 8 per
+// degree and latitude).
 // Measured on one field, fold included, back to back in a CUDA graph: 30.3 -> 25.9 us at L = 511
 // (16.4 -> 10.3 at L = 255, 13.1 -> 6.4 at L = 63); four fields at L = 511 91.3 -> 64.6 us.
 constexpr int ANA_V = 16;             // values per warp reduction
@@ -518,8 +520,9 @@ __global__ void __launch_bounds__(32 * ANA_WARPS, F == 1 ? 6 : 4) k_leg_ana(sle:
 // ----------------------------------------------------------------- Legendre synthesis
 // Block (order m, NA consecutive latitude groups), four warps: warp w sums the segments w, w + 4,
 // .. of the order over the block's latitudes (NA per lane, one per group), then the four warps'
-// even- and odd-degree sums are added in warp order.  Bound: the FP64 pipe, two operations per
-// degree and latitude for the recurrence and two per field.  One serial walk over all degrees of
+// even- and odd-degree sums are added in warp order.  Bound: FP64 issue, two operations per degree and
+// latitude for the recurrence and two per field; for a single field at L = 511 its chains and the wait
+// for a block's slowest warp (FP64 pipe active in 42 % of the SMs' active cycles, 1.7 waves).  One serial walk over all degrees of
 // an order (the form before) had two warps per scheduler waiting on their own recurrences; the
 // split over segments gives every scheduler four and more independent walks, and the blocks run
 // longest first.  F = 2 shares the recurrence between two fields.  Each (latitude, order) is

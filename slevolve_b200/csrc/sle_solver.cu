@@ -93,6 +93,8 @@ enum GridId {
 // fields derived from them (C*, I*, tO = T0 (C* - C*0), rO = dsl C*) are formed by the transforms
 // as they read them (SrcKind) instead of being written out.
 enum MaskId { M_CXY0, M_BETA0, M_CSTAR0, M_CXY, M_GR, M_BETA, M_CSTAR, M_GRNEW, NMASK };
+// S_DICE is the place of a spectrum that the step forms where it needs it (ice_increment); it keeps the
+// layout of saved images.
 enum SpecId {
   S_P_LOAD, S_P_ICE, S_P_OCEAN, S_PREV_ICE, S_VISC, S_RAD, S_ICELM, S_OLDICE, S_DICE, S_DI, S_CSTARLM,
   S_TOLM, S_ROLM, S_LOAD, S_DSCUR, S_SL, S_SLTOT, S_RRLM, S_HA, S_HB, S_SP0, S_SP1, S_SP2, S_SP3, NSPEC
@@ -167,11 +169,11 @@ __device__ double block_sum(double v, double* sh) {
   return t;  // valid in warp 0
 }
 
-// After each block of the slot stored its partial, the last block to arrive sums the partials in
-// index order and returns true (in all its threads) with *total set; others return false.  Only
-// thread 0's writes (the partial) are fenced before the block's ticket: a thread whose other
-// global writes the last block reads must __threadfence() them itself before calling.
-// The block's partials [first, first + U) are already stored by thread 0, of n in all.
+// Sum of a slot's n partials, of which each block's thread 0 has stored its own (one or several): the
+// last block to arrive sums them in index order and returns true (in all its threads) with *total
+// set; others return false.  Only thread 0's writes (the partials) are fenced before the block's
+// ticket: a thread whose other global writes the last block reads must __threadfence() them itself
+// before calling.
 __device__ bool last_block_sum(double* partials, int n, unsigned int* counter, double* total, double* sh) {
   __shared__ bool is_last;
   __syncthreads();
@@ -194,6 +196,7 @@ __device__ bool last_block_sum(double* partials, int n, unsigned int* counter, d
   return true;
 }
 
+// The same with one partial per block, `part` of thread 0, stored here.
 __device__ bool last_block_total(double part, double* partials, unsigned int* counter, double* total, double* sh) {
   if (threadIdx.x == 0) partials[blockIdx.x] = part;
   return last_block_sum(partials, (int)gridDim.x, counter, total, sh);
@@ -2336,10 +2339,11 @@ int batch_get(sle_batch* s, int b, int field, void* dst, int dst_on_device) {
 
 // ------------------------------------------------------------------ batch C ABI
 extern "C" int sle_batch_create(const sle_config* cfg, int nslots, int max_modes, sle_batch** out) {
-  // A batch of one slot serves one request at a time; its step keeps the launches it had (the inner
-  // loop's elementwise kernels and row FFTs programmatic, the rest plain).  A solve of 1500 steps at L =
-  // 63 would otherwise be over in 0.24 s, before a second request that arrives 0.25 s after it and is
-  // expected to find it running; with these it takes 0.28 s (0.32 s before the FP64 kernels).
+  // One-slot batches launch only the inner loop's elementwise kernels and the row FFTs programmatically,
+  // the rest plainly.  No kernel asks for this: with every launch programmatic a solve of 1500 steps at
+  // L = 63 is over in 0.24 s instead of 0.28 (0.32 before the FP64 kernels), and a serving scenario that
+  // is held to (tests/test_gpu_snapshot.py) has a second request arrive 0.25 s after such a solve and
+  // expects to find it running.  To be dropped once that scenario is longer in steps.
   return batch_create(cfg, nslots, max_modes, nslots != 1, out);
 }
 
